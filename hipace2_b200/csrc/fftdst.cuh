@@ -21,14 +21,6 @@ struct Cx {
     R re, im;
 };
 
-// rows per block by transform length (shared memory: RB/2 complex arrays of M elements); passes
-// with fewer than 2 blocks per SM at that size run 2 rows per block instead
-template <int M>
-struct DstCfg {
-    static constexpr int RB = M <= 2048 ? 4 : 2;
-};
-constexpr int kDstSmallRows = 2 * 148 * 4;  // rows below which a pass uses 2 rows per block
-
 template <class R>
 __device__ __forceinline__ Cx<R> cmul(const Cx<R>& v0, const Cx<R>& w) {
     return {v0.re * w.re - v0.im * w.im, v0.re * w.im + v0.im * w.re};
@@ -87,104 +79,244 @@ __device__ __forceinline__ void fft_block(Cx<R>* z, int nfft, const Cx<R>* __res
     (void)s;
 }
 
-template <int LOGM>
-__device__ __forceinline__ int brev(int j) {
-    return (int)(__brev((unsigned)j) >> (32 - LOGM));
+// ------------------------------------------------------------------------------------------
+// The transform of a row pair: FFT of length M = 2(n+1) with 8 elements per thread in registers
+// (Stockham autosort: radix-8 passes, then one of radix 8, 4 or 2), so that M = 2048 passes
+// through shared memory 3 times; the in-place radix-2/4 form it replaces did 6 times and
+// put its input in bit-reversed order first. Bound by shared memory and, in double, the FP64
+// pipe; a 1023^2 solve of three fields took 469 us (double) and 323 us (single) with that form.
+// ------------------------------------------------------------------------------------------
+// row pairs per block: blocks of at least 64 threads, four rows per block up to M = 2048 so that a
+// transposed write covers 32 bytes in double
+template <int M>
+struct DstCfg {
+    static constexpr int T = M / 8;                                   // threads per row pair
+    static constexpr int F = M <= 256 ? 64 / T * 2 : M <= 2048 ? 2 : 1;  // row pairs per block
+    static constexpr int RB = 2 * F;
+    static constexpr int NT = F * T;
+    static constexpr int MP = M + M / 8;                              // padded complex row
+    template <class R>
+    static constexpr size_t smem() { return (size_t)F * MP * sizeof(Cx<R>); }
+};
+// one word group of padding per 8 elements: the stride-8 writes of the first pass then touch
+// different banks
+__device__ __forceinline__ int dst_pad(int i) { return i + (i >> 3); }
+
+// 8-point DFT (exp(-i)) in place, outputs in natural order
+template <class R>
+__device__ __forceinline__ void dft8(Cx<R> (&v)[8]) {
+    const R h = R(0.70710678118654752440);
+    auto bf = [](Cx<R>& a, Cx<R>& b) {
+        const Cx<R> t = {a.re - b.re, a.im - b.im};
+        a = {a.re + b.re, a.im + b.im};
+        b = t;
+    };
+    bf(v[0], v[4]); bf(v[1], v[5]); bf(v[2], v[6]); bf(v[3], v[7]);
+    // odd half times exp(-i pi q / 4)
+    v[5] = {(v[5].re + v[5].im) * h, (v[5].im - v[5].re) * h};
+    v[6] = {v[6].im, -v[6].re};
+    v[7] = {(v[7].im - v[7].re) * h, -(v[7].re + v[7].im) * h};
+    bf(v[0], v[2]); bf(v[1], v[3]); bf(v[4], v[6]); bf(v[5], v[7]);
+    v[3] = {v[3].im, -v[3].re};
+    v[7] = {v[7].im, -v[7].re};
+    bf(v[0], v[1]); bf(v[2], v[3]); bf(v[4], v[5]); bf(v[6], v[7]);
+    // v[bit-reversed] -> natural order
+    Cx<R> t = v[1]; v[1] = v[4]; v[4] = t;
+    t = v[3]; v[3] = v[6]; v[6] = t;
+}
+template <class R>
+__device__ __forceinline__ void dft4(Cx<R>& a, Cx<R>& b, Cx<R>& c, Cx<R>& d) {
+    const Cx<R> s0 = {a.re + c.re, a.im + c.im}, d0 = {a.re - c.re, a.im - c.im};
+    const Cx<R> s1 = {b.re + d.re, b.im + d.im}, d1 = {b.im - d.im, d.re - b.re};  // -i (b - d)
+    a = {s0.re + s1.re, s0.im + s1.im};
+    b = {d0.re + d1.re, d0.im + d1.im};
+    c = {s0.re - s1.re, s0.im - s1.im};
+    d = {d0.re - d1.re, d0.im - d1.im};
 }
 
-// odd extension of row values (val(row, e), e in [0, n)) into bit-reversed order
-template <class R, int M, int LOGM, class Get>
-__device__ __forceinline__ void load_odd(Cx<R>* z, int nfft, int n, Get get) {
-    for (int t = threadIdx.x; t < nfft * M; t += blockDim.x) {
-        const int f = t / M, j = t - f * M;
-        R re = 0, im = 0;
-        if (j >= 1 && j <= n) { re = get(2 * f, j - 1); im = get(2 * f + 1, j - 1); }
-        else if (j >= n + 2) { re = -get(2 * f, M - j - 1); im = -get(2 * f + 1, M - j - 1); }
-        z[f * M + brev<LOGM>(j)] = {re, im};
+// FFT of one row pair by the M/8 threads t: on entry v[q] = x[t + q M/8], on return v[q] = X[t + q M/8].
+// z: the pair's padded row of shared memory; the whole block calls.
+template <class R, int M, int LOGM>
+__device__ __forceinline__ void fft_regs(Cx<R> (&v)[8], Cx<R>* z, int t, const Cx<R>* __restrict__ tw) {
+    constexpr int T = M / 8;
+    dft8(v);
+    __syncthreads();  // (the row may still be read by the previous use)
+#pragma unroll
+    for (int q = 0; q < 8; ++q) z[dst_pad(8 * t + q)] = v[q];
+    __syncthreads();
+    int l = 8;
+    constexpr int full = LOGM / 3, rest = LOGM % 3;  // radix-8 passes, log2 of the last radix (0: none)
+#pragma unroll
+    for (int p = 1; p < full; ++p) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = z[dst_pad(t + q * T)];
+        const int k = t & (l - 1), u = k * (M / (8 * l));
+        const Cx<R> w1 = tw[u], w2 = tw[2 * u], w4 = tw[4 * u], w3 = cmul(w1, w2);
+        v[1] = cmul(v[1], w1); v[2] = cmul(v[2], w2); v[3] = cmul(v[3], w3); v[4] = cmul(v[4], w4);
+        v[5] = cmul(v[5], cmul(w1, w4)); v[6] = cmul(v[6], cmul(w2, w4)); v[7] = cmul(v[7], cmul(w3, w4));
+        dft8(v);
+        if (p + 1 < full || rest) {
+            __syncthreads();
+            const int o = (t - k) * 8 + k;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) z[dst_pad(o + q * l)] = v[q];
+            __syncthreads();
+        }
+        l *= 8;
+    }
+    if constexpr (rest == 2) {
+        // radix 4, l = M/4: butterflies t and t + M/8
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = z[dst_pad(t + q * T)];
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            const int k = t + s * T;
+            const Cx<R> w1 = tw[k], w2 = tw[2 * k];
+            v[s + 2] = cmul(v[s + 2], w1);
+            v[s + 4] = cmul(v[s + 4], w2);
+            v[s + 6] = cmul(v[s + 6], cmul(w1, w2));
+            dft4(v[s], v[s + 2], v[s + 4], v[s + 6]);
+        }
+    } else if constexpr (rest == 1) {
+        // radix 2, l = M/2: butterflies t + s M/8
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = z[dst_pad(t + q * T)];
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const Cx<R> a = v[s], b = cmul(v[s + 4], tw[t + s * T]);
+            v[s] = {a.re + b.re, a.im + b.im};
+            v[s + 4] = {a.re - b.re, a.im - b.im};
+        }
+    }
+}
+
+// odd extension of the row pair (get(0 / 1, e), e in [0, n)) as complex elements t + q M/8
+template <class R, int M, class Get>
+__device__ __forceinline__ void load_odd(Cx<R> (&v)[8], int t, int n, Get get) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int j = t + q * (M / 8);
+        if (q < 4) v[q] = j >= 1 ? Cx<R>{get(0, j - 1), get(1, j - 1)} : Cx<R>{R(0), R(0)};
+        else v[q] = j > n + 1 ? Cx<R>{-get(0, M - j - 1), -get(1, M - j - 1)} : Cx<R>{R(0), R(0)};
+    }
+}
+
+// The rows of a block written transposed: out[(plane n + e) rows_per_plane + row], through shared
+// memory so that the block's rows of one e are written together. v[q < 4] holds elements
+// t + q M/8 - 1 of the pair f.
+template <class R, int M>
+__device__ __forceinline__ void store_transposed(const Cx<R> (&v)[8], Cx<R>* smem, int f, int t, int r0, int nrows, int n,
+                                                 int rows_per_plane, R* __restrict__ out) {
+    using C = DstCfg<M>;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int j = t + q * (M / 8);
+        // DST-I of the pair: row 0 is -Im / 2, row 1 is Re / 2
+        smem[(size_t)j * C::F + f] = {v[q].im * R(-0.5), v[q].re * R(0.5)};
     }
     __syncthreads();
+    const R* s = reinterpret_cast<const R*>(smem);
+    static_assert(C::NT % C::RB == 0, "a thread writes one row");
+    const int r = threadIdx.x % C::RB, row = r0 + r;
+    if (row >= nrows) return;
+    const int pl = row / rows_per_plane, rr = row - pl * rows_per_plane;
+    R* o = out + (size_t)pl * n * rows_per_plane + rr;
+    for (int e = threadIdx.x / C::RB; e < n; e += C::NT / C::RB) o[(size_t)e * rows_per_plane] = s[(e + 1) * C::RB + r];
 }
 
-// DST-I value of element e of block row r after the FFT
-template <class R, int M>
-__device__ __forceinline__ R dst_val(const Cx<R>* z, int r, int e) {
-    const Cx<R> v = z[(r >> 1) * M + e + 1];
-    return (r & 1) ? v.re * R(0.5) : -v.im * R(0.5);
-}
-
-// Pass over rows: out(row, e) = DST-I(in row)[e]; written transposed:
+// Pass over rows: DST-I of every row of length n, written transposed:
 // out[(row / rows_per_plane) * n * rows_per_plane + e * rows_per_plane + row % rows_per_plane]
-template <class R, int M, int LOGM, int RB>
-__global__ void __launch_bounds__(256) k_dst_pass_t(const R* __restrict__ in, int nrows, int n, int rows_per_plane,
-                                                    R* __restrict__ out, const Cx<R>* __restrict__ tw) {
+template <class R, int M, int LOGM>
+__global__ void __launch_bounds__(DstCfg<M>::NT, 1024 / DstCfg<M>::NT) k_dst_pass_t(const R* __restrict__ in, int nrows, int n,
+                                                              int rows_per_plane, R* __restrict__ out,
+                                                              const Cx<R>* __restrict__ tw) {
     HPQ_PDL_ENTRY();
-    extern __shared__ unsigned char smem_raw[];
-    Cx<R>* z = reinterpret_cast<Cx<R>*>(smem_raw);
-    const int r0 = blockIdx.x * RB;
-    auto get = [&](int r, int e) -> R { const int row = r0 + r; return row < nrows ? in[(size_t)row * n + e] : R(0); };
-    load_odd<R, M, LOGM>(z, RB / 2, n, get);
-    fft_block<R, M, LOGM>(z, RB / 2, tw);
-    for (int t = threadIdx.x; t < RB * n; t += blockDim.x) {
-        const int r = t % RB, e = t / RB;
-        const int row = r0 + r;
-        if (row >= nrows) continue;
-        const int pl = row / rows_per_plane, rr = row - pl * rows_per_plane;
-        out[((size_t)pl * n + e) * rows_per_plane + rr] = dst_val<R, M>(z, r, e);
-    }
+    using C = DstCfg<M>;
+    extern __shared__ __align__(16) unsigned char dst_smem[];
+    Cx<R>* z = reinterpret_cast<Cx<R>*>(dst_smem);
+    const int f = threadIdx.x / C::T, t = threadIdx.x % C::T, r0 = blockIdx.x * C::RB, row0 = r0 + 2 * f;
+    auto get = [&](int r, int e) -> R { return row0 + r < nrows ? in[(size_t)(row0 + r) * n + e] : R(0); };
+    Cx<R> v[8];
+    load_odd<R, M>(v, t, n, get);
+    fft_regs<R, M, LOGM>(v, z + f * C::MP, t, tw);
+    store_transposed<R, M>(v, z, f, t, r0, nrows, n, rows_per_plane, out);
 }
 
 // y-pass, eigenvalue multiply, y-pass; rows are (plane, i) of length n = ny; eig is [j][i] with
-// row length nxe; written transposed back to [plane][j][i]
-template <class R, int M, int LOGM, int RB>
-__global__ void __launch_bounds__(256) k_dst_pass_eig(const R* __restrict__ in, int nrows, int n, int rows_per_plane,
-                                                      const R* __restrict__ eig, R* __restrict__ out,
-                                                      const Cx<R>* __restrict__ tw) {
-    HPQ_PDL_ENTRY();
-    extern __shared__ unsigned char smem_raw[];
-    Cx<R>* z = reinterpret_cast<Cx<R>*>(smem_raw);
-    R* tmp = reinterpret_cast<R*>(z + (RB / 2) * M);
-    const int r0 = blockIdx.x * RB;
-    auto get = [&](int r, int e) -> R { const int row = r0 + r; return row < nrows ? in[(size_t)row * n + e] : R(0); };
-    load_odd<R, M, LOGM>(z, RB / 2, n, get);
-    fft_block<R, M, LOGM>(z, RB / 2, tw);
-    for (int t = threadIdx.x; t < RB * n; t += blockDim.x) {
-        const int r = t / n, e = t - r * n;
-        const int row = r0 + r;
-        const int i = row % rows_per_plane;
-        tmp[t] = row < nrows ? dst_val<R, M>(z, r, e) * eig[(size_t)e * rows_per_plane + i] : R(0);
+// row length rows_per_plane; written transposed back to [plane][j][i]
+template <class R, int M, int LOGM, class Eig>
+__device__ __forceinline__ void dst_pass_eig(const R* __restrict__ in, int nrows, int n, int rows_per_plane, Eig eig,
+                                             R* __restrict__ out, const Cx<R>* __restrict__ tw) {
+    using C = DstCfg<M>;
+    extern __shared__ __align__(16) unsigned char dst_smem[];
+    Cx<R>* z = reinterpret_cast<Cx<R>*>(dst_smem);
+    const int f = threadIdx.x / C::T, t = threadIdx.x % C::T, r0 = blockIdx.x * C::RB, row0 = r0 + 2 * f;
+    auto get = [&](int r, int e) -> R { return row0 + r < nrows ? in[(size_t)(row0 + r) * n + e] : R(0); };
+    Cx<R> v[8];
+    load_odd<R, M>(v, t, n, get);
+    Cx<R>* zf = z + f * C::MP;
+    fft_regs<R, M, LOGM>(v, zf, t, tw);
+    // odd extension of the products; elements beyond M/2 are those of the mirrored thread
+    const int i0 = row0 % rows_per_plane, i1 = (row0 + 1) % rows_per_plane;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int j = t + q * (M / 8);
+        Cx<R> w{R(0), R(0)};
+        if (j >= 1) {
+            w.re = row0 < nrows ? v[q].im * R(-0.5) * eig(j - 1, i0) : R(0);
+            w.im = row0 + 1 < nrows ? v[q].re * R(0.5) * eig(j - 1, i1) : R(0);
+        }
+        v[q] = w;
+        zf[j] = w;
     }
     __syncthreads();
-    auto get2 = [&](int r, int e) -> R { return tmp[r * n + e]; };
-    load_odd<R, M, LOGM>(z, RB / 2, n, get2);
-    fft_block<R, M, LOGM>(z, RB / 2, tw);
-    for (int t = threadIdx.x; t < RB * n; t += blockDim.x) {
-        const int r = t % RB, e = t / RB;
-        const int row = r0 + r;
-        if (row >= nrows) continue;
-        const int pl = row / rows_per_plane, rr = row - pl * rows_per_plane;
-        out[((size_t)pl * n + e) * rows_per_plane + rr] = dst_val<R, M>(z, r, e);
+#pragma unroll
+    for (int q = 4; q < 8; ++q) {
+        const int j = t + q * (M / 8);
+        const Cx<R> w = j > M / 2 ? zf[M - j] : Cx<R>{R(0), R(0)};
+        v[q] = {-w.re, -w.im};
     }
+    // (the twiddles are read again: kept over the first transform they cost 60 registers in double)
+    asm volatile("" : "+l"(tw));
+    fft_regs<R, M, LOGM>(v, zf, t, tw);
+    store_transposed<R, M>(v, z, f, t, r0, nrows, n, rows_per_plane, out);
+}
+template <class R, int M, int LOGM>
+__global__ void __launch_bounds__(DstCfg<M>::NT, 1024 / DstCfg<M>::NT) k_dst_pass_eig(const R* __restrict__ in, int nrows, int n,
+                                                                int rows_per_plane, const R* __restrict__ eig,
+                                                                R* __restrict__ out, const Cx<R>* __restrict__ tw) {
+    HPQ_PDL_ENTRY();
+    dst_pass_eig<R, M, LOGM>(in, nrows, n, rows_per_plane,
+                             [&](int e, int i) { return eig[(size_t)e * rows_per_plane + i]; }, out, tw);
 }
 
 // final x-pass: rows are (plane k, j) of length nx; result scattered into field component comp[k]
-template <class R, int M, int LOGM, int RB>
-__global__ void __launch_bounds__(256) k_dst_pass_field(const R* __restrict__ in, int nrows, int n, int ny, R* base,
-                                                        size_t cstride, int pitch, int c0, int c1, int c2,
-                                                        const Cx<R>* __restrict__ tw) {
+template <class R, int M, int LOGM>
+__global__ void __launch_bounds__(DstCfg<M>::NT, 1024 / DstCfg<M>::NT) k_dst_pass_field(const R* __restrict__ in, int nrows, int n, int ny,
+                                                                  R* base, size_t cstride, int pitch, int c0, int c1,
+                                                                  int c2, const Cx<R>* __restrict__ tw) {
     HPQ_PDL_ENTRY();
-    extern __shared__ unsigned char smem_raw[];
-    Cx<R>* z = reinterpret_cast<Cx<R>*>(smem_raw);
-    const int r0 = blockIdx.x * RB;
-    auto get = [&](int r, int e) -> R { const int row = r0 + r; return row < nrows ? in[(size_t)row * n + e] : R(0); };
-    load_odd<R, M, LOGM>(z, RB / 2, n, get);
-    fft_block<R, M, LOGM>(z, RB / 2, tw);
-    for (int t = threadIdx.x; t < RB * n; t += blockDim.x) {
-        const int r = t / n, e = t - r * n;
-        const int row = r0 + r;
+    using C = DstCfg<M>;
+    extern __shared__ __align__(16) unsigned char dst_smem[];
+    Cx<R>* z = reinterpret_cast<Cx<R>*>(dst_smem);
+    const int f = threadIdx.x / C::T, t = threadIdx.x % C::T, row0 = blockIdx.x * C::RB + 2 * f;
+    auto get = [&](int r, int e) -> R { return row0 + r < nrows ? in[(size_t)(row0 + r) * n + e] : R(0); };
+    Cx<R> v[8];
+    load_odd<R, M>(v, t, n, get);
+    fft_regs<R, M, LOGM>(v, z + f * C::MP, t, tw);
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const int row = row0 + r;
         if (row >= nrows) continue;
         const int k = row / ny, j = row - k * ny;
-        const int comp = k == 0 ? c0 : (k == 1 ? c1 : c2);
-        base[(size_t)comp * cstride + (size_t)(j + kGuardAlloc) * pitch + (e + kGuardAlloc)] = dst_val<R, M>(z, r, e);
+        R* o = base + (size_t)(k == 0 ? c0 : (k == 1 ? c1 : c2)) * cstride + (size_t)(j + kGuardAlloc) * pitch + kGuardAlloc;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int i = t + q * (M / 8);
+            if (i >= 1) o[i - 1] = r ? v[q].re * R(0.5) : v[q].im * R(-0.5);
+        }
     }
 }
 
@@ -474,55 +606,34 @@ public:
                    nrhs > 2 ? comps[2] : comps[0], A);
         HPQ_LAUNCH_CHECK();
     }
-    template <int M, int RB>
-    static size_t smem_fft() { return (size_t)(RB / 2) * M * sizeof(Cx<R>); }
-    template <int M, int RB>
-    static size_t smem_eig(int n) { return smem_fft<M, RB>() + (size_t)RB * n * sizeof(R); }
-    template <int M, int LOGM, int RB>
-    static void set_attrs_rb() {
-        const int big = 200 * 1024;
-        HPQ_CUDA(cudaFuncSetAttribute(k_dst_pass_t<R, M, LOGM, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-        HPQ_CUDA(cudaFuncSetAttribute(k_dst_pass_eig<R, M, LOGM, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-        HPQ_CUDA(cudaFuncSetAttribute(k_dst_pass_field<R, M, LOGM, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    }
     template <int M, int LOGM>
     static void set_attrs() {
-        set_attrs_rb<M, LOGM, DstCfg<M>::RB>();
-        if (DstCfg<M>::RB != 2) set_attrs_rb<M, LOGM, 2>();
+        const int smem = (int)DstCfg<M>::template smem<R>();
+        HPQ_CUDA(cudaFuncSetAttribute(k_dst_pass_t<R, M, LOGM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        HPQ_CUDA(cudaFuncSetAttribute(k_dst_pass_eig<R, M, LOGM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        HPQ_CUDA(cudaFuncSetAttribute(k_dst_pass_field<R, M, LOGM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     }
-
-    template <int M, int LOGM, int RB>
-    void pass_t_rb(cudaStream_t st, const R* in, int nrows, int n, int rpp, R* out, const Cx<R>* tw) {
-        hpq_launch(k_dst_pass_t<R, M, LOGM, RB>, dim3((nrows + RB - 1) / RB), dim3(256), smem_fft<M, RB>(), st, in, nrows, n, rpp, out, tw);
-        HPQ_LAUNCH_CHECK();
-    }
+    template <int M>
+    static dim3 dst_grid(int nrows) { return dim3((nrows + DstCfg<M>::RB - 1) / DstCfg<M>::RB); }
     template <int M, int LOGM>
     void pass_t(cudaStream_t st, const R* in, int nrows, int n, int rpp, R* out, const Cx<R>* tw) {
-        if (nrows < kDstSmallRows) pass_t_rb<M, LOGM, 2>(st, in, nrows, n, rpp, out, tw);
-        else pass_t_rb<M, LOGM, DstCfg<M>::RB>(st, in, nrows, n, rpp, out, tw);
-    }
-    template <int M, int LOGM, int RB>
-    void pass_eig_rb(cudaStream_t st, const R* in, int nrows, int n, int rpp, const R* eig, R* out, const Cx<R>* tw) {
-        hpq_launch(k_dst_pass_eig<R, M, LOGM, RB>, dim3((nrows + RB - 1) / RB), dim3(256), smem_eig<M, RB>(n), st, in, nrows, n, rpp, eig, out, tw);
+        using C = DstCfg<M>;
+        hpq_launch(k_dst_pass_t<R, M, LOGM>, dst_grid<M>(nrows), dim3(C::NT), C::template smem<R>(), st, in, nrows, n, rpp, out, tw);
         HPQ_LAUNCH_CHECK();
     }
     template <int M, int LOGM>
     void pass_eig(cudaStream_t st, const R* in, int nrows, int n, int rpp, const R* eig, R* out, const Cx<R>* tw) {
-        if (nrows < kDstSmallRows) pass_eig_rb<M, LOGM, 2>(st, in, nrows, n, rpp, eig, out, tw);
-        else pass_eig_rb<M, LOGM, DstCfg<M>::RB>(st, in, nrows, n, rpp, eig, out, tw);
-    }
-    template <int M, int LOGM, int RB>
-    void pass_field_rb(cudaStream_t st, const R* in, int nrows, int n, R* base, size_t cs, int pitch, const int* comps,
-                       int nrhs, const Cx<R>* tw) {
-        hpq_launch(k_dst_pass_field<R, M, LOGM, RB>, dim3((nrows + RB - 1) / RB), dim3(256), smem_fft<M, RB>(), st,
-            in, nrows, n, ny, base, cs, pitch, comps[0], nrhs > 1 ? comps[1] : comps[0], nrhs > 2 ? comps[2] : comps[0], tw);
+        using C = DstCfg<M>;
+        hpq_launch(k_dst_pass_eig<R, M, LOGM>, dst_grid<M>(nrows), dim3(C::NT), C::template smem<R>(), st, in, nrows, n, rpp, eig, out, tw);
         HPQ_LAUNCH_CHECK();
     }
     template <int M, int LOGM>
     void pass_field(cudaStream_t st, const R* in, int nrows, int n, R* base, size_t cs, int pitch, const int* comps,
                     int nrhs, const Cx<R>* tw) {
-        if (nrows < kDstSmallRows) pass_field_rb<M, LOGM, 2>(st, in, nrows, n, base, cs, pitch, comps, nrhs, tw);
-        else pass_field_rb<M, LOGM, DstCfg<M>::RB>(st, in, nrows, n, base, cs, pitch, comps, nrhs, tw);
+        using C = DstCfg<M>;
+        hpq_launch(k_dst_pass_field<R, M, LOGM>, dst_grid<M>(nrows), dim3(C::NT), C::template smem<R>(), st,
+            in, nrows, n, ny, base, cs, pitch, comps[0], nrhs > 1 ? comps[1] : comps[0], nrhs > 2 ? comps[2] : comps[0], tw);
+        HPQ_LAUNCH_CHECK();
     }
 
 #define HPQ_DST_DISPATCH(Mval, CALL)                       \

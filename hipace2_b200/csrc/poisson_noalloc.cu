@@ -4,9 +4,9 @@
 // being captured into a graph (allocation is not a capturable operation), plugins of host
 // frameworks that own the device memory pool and forbid side allocations, and real-time loops
 // that must not pay for or fail on an allocation at solve time. This entry point serves them:
-// the caller passes the right-hand side and the solution buffer; the temporaries of the solve
-// (the transformed intermediate, the eigenvalues and the FFT twiddles) live in one file-scope
-// device array of fixed size. CUDA loads the library's device code lazily, so the array's
+// the caller passes the right-hand side and the solution buffer; the transformed intermediate of
+// the solve lives in one file-scope device array of fixed size (the FFT twiddles of every length in
+// another, filled when the device is set up; the eigenvalues are formed where they are used). CUDA loads the library's device code lazily, so the array's
 // memory is committed on a device by the first call on that device (which can therefore fail
 // with HPQ_ERR_CUDA when the device is already full) and held until the process exits.
 //
@@ -21,6 +21,7 @@
 // is made.
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <mutex>
 
 #include "../../include/hpq.h"
@@ -30,21 +31,35 @@ namespace {
 
 constexpr int kMaxN = 1023;
 constexpr size_t kPlane = (size_t)kMaxN * kMaxN;          // one nx x ny plane
-constexpr size_t kTw = 2048;                               // complex twiddles: M/2 for x and y
-constexpr size_t kScratchDoubles = 2 * kPlane + 2 * kTw;   // work plane, eigenvalues, twiddles
+constexpr size_t kTw = 2048;                               // complex twiddles of M = 64 .. 2048, M/2 each
+constexpr size_t kScratchDoubles = 2 * kPlane + 2 * kTw;   // work plane (the rest is not used)
 
 static __device__ __align__(256) double g_poisson_scratch[kScratchDoubles];
+static __device__ __align__(256) double g_poisson_twiddles[2 * kTw];
 
 constexpr int kMaxDevices = 64;
 std::mutex g_mutex;
 double* g_scratch_ptr[kMaxDevices] = {};
+const hpq::Cx<double>* g_twiddle_ptr[kMaxDevices] = {};
 
 cudaError_t set_smem_attributes();
 
 // Set-up, once per device with that device current: the host address of the array is only a
 // stand-in, kernels must be given the device address returned here. The shared-memory limits of
-// the pass kernels are raised at the same time, so later calls make no set-up call at all.
-int scratch_for_current_device(double** out) {
+// the pass kernels are raised and the twiddles written at the same time, so later calls make no
+// set-up call at all.
+size_t tw_offset(int M) { return (size_t)M / 2 - 32; }  // 32 + 64 + .. + M/4 before length M
+cudaError_t fill_twiddles(void* dst) {
+    static double h[2 * kTw];  // (under the mutex)
+    const double pi = 3.14159265358979323846;
+    for (int M = 64; M <= 2048; M *= 2)
+        for (int k = 0; k < M / 2; ++k) {
+            h[2 * (tw_offset(M) + k)] = std::cos(2 * pi * k / M);
+            h[2 * (tw_offset(M) + k) + 1] = -std::sin(2 * pi * k / M);
+        }
+    return cudaMemcpy(dst, h, sizeof(h), cudaMemcpyHostToDevice);
+}
+int scratch_for_current_device(double** out, const hpq::Cx<double>** tw) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return HPQ_ERR_CUDA;
     std::lock_guard<std::mutex> lock(g_mutex);
@@ -52,49 +67,41 @@ int scratch_for_current_device(double** out) {
         void* p = nullptr;
         if (cudaGetSymbolAddress(&p, g_poisson_scratch) != cudaSuccess || !p) return HPQ_ERR_CUDA;
         if (set_smem_attributes() != cudaSuccess) return HPQ_ERR_CUDA;
+        void* t = nullptr;
+        if (cudaGetSymbolAddress(&t, g_poisson_twiddles) != cudaSuccess || !t) return HPQ_ERR_CUDA;
+        if (fill_twiddles(t) != cudaSuccess) return HPQ_ERR_CUDA;
+        g_twiddle_ptr[dev] = static_cast<const hpq::Cx<double>*>(t);
         g_scratch_ptr[dev] = static_cast<double*>(p);
     }
     *out = g_scratch_ptr[dev];
+    *tw = g_twiddle_ptr[dev];
     return HPQ_OK;
 }
 
-// eigenvalues of the 5-point Laplacian with the normalisation of the two DST-I per axis
-__global__ void k_fill_eig(double* eig, int nx, int ny, double dx, double dy) {
-    const double pi = 3.14159265358979323846;
-    const double sxf = pi / (2. * (nx + 1)), syf = pi / (2. * (ny + 1));
+// y-pass, division by the eigenvalues of the 5-point Laplacian (with the normalisation of the two
+// DST-I per axis), y-pass. The eigenvalues are separable: a thread needs the sines of its two rows and
+// four columns, where a table of nx * ny took a kernel of its own and two sines per point.
+template <int M, int LOGM>
+__global__ void __launch_bounds__(hpq::DstCfg<M>::NT, 1024 / hpq::DstCfg<M>::NT) k_pass_eig(const double* __restrict__ in, int nx, int ny, double dx,
+                                                                 double dy, double* __restrict__ out,
+                                                                 const hpq::Cx<double>* __restrict__ tw) {
+    HPQ_PDL_ENTRY();
     const double norm = (2.0 / (nx + 1)) * (2.0 / (ny + 1));
-    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < (long long)nx * ny;
-         k += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(k % nx), j = (int)(k / nx);
-        double a = sin((i + 1) * sxf), b = sin((j + 1) * syf);
-        a *= a;
-        b *= b;
-        eig[k] = norm / (-4.0 * (a / (dx * dx) + b / (dy * dy)));
-    }
+    auto lambda = [](int k, int n, double h) {
+        const double s = sinpi((k + 1) / (2.0 * (n + 1)));
+        return s * s / (h * h);
+    };
+    hpq::dst_pass_eig<double, M, LOGM>(
+        in, nx, ny, nx, [&](int e, int i) { return norm / (-4.0 * (lambda(i, nx, dx) + lambda(e, ny, dy))); }, out, tw);
 }
-
-__global__ void k_fill_twiddles(hpq::Cx<double>* tw, int M) {
-    const double pi = 3.14159265358979323846;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < M / 2; k += gridDim.x * blockDim.x)
-        tw[k] = {cos(2 * pi * k / M), -sin(2 * pi * k / M)};
-}
-
-// shared memory of one block of a pass: rb/2 complex rows of length M (the eigenvalue pass adds
-// rb rows of n <= kMaxN reals)
-template <int M>
-constexpr size_t smem_t() { return (size_t)(hpq::DstCfg<M>::RB / 2) * M * sizeof(hpq::Cx<double>); }
 
 template <int M, int LOGM>
 cudaError_t set_attrs_for() {
-    constexpr int RB = hpq::DstCfg<M>::RB;
-    cudaError_t e = cudaFuncSetAttribute(hpq::k_dst_pass_t<double, M, LOGM, RB>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t<M>());
+    const int smem = (int)hpq::DstCfg<M>::template smem<double>();
+    cudaError_t e = cudaFuncSetAttribute(hpq::k_dst_pass_t<double, M, LOGM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_pass_eig<M, LOGM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(hpq::k_dst_pass_eig<double, M, LOGM, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(smem_t<M>() + (size_t)RB * kMaxN * sizeof(double)));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(hpq::k_dst_pass_field<double, M, LOGM, RB>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t<M>());
+        e = cudaFuncSetAttribute(hpq::k_dst_pass_field<double, M, LOGM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     return e;
 }
 
@@ -108,36 +115,42 @@ cudaError_t set_smem_attributes() {
     return e;
 }
 
+// Launch of one pass; a dependent one may start before the pass in front of it has ended (its
+// prologue waits for that pass)
+template <int M, class... K, class... A>
+cudaError_t launch(void (*kernel)(K...), cudaStream_t st, int nrows, bool dependent, A... args) {
+    using C = hpq::DstCfg<M>;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((nrows + C::RB - 1) / C::RB);
+    cfg.blockDim = dim3(C::NT);
+    cfg.dynamicSmemBytes = C::template smem<double>();
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = dependent && hpq::pdl_enabled() ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 template <int M, int LOGM>
 cudaError_t pass_t(cudaStream_t st, const double* in, int nrows, int n, int rpp, double* out,
                    const hpq::Cx<double>* tw) {
-    const int rb = hpq::DstCfg<M>::RB;
-    const size_t smem = smem_t<M>();
-    hpq::k_dst_pass_t<double, M, LOGM, hpq::DstCfg<M>::RB><<<(nrows + rb - 1) / rb, 256, smem, st>>>(in, nrows, n, rpp, out, tw);
-    return cudaGetLastError();
+    return launch<M>(hpq::k_dst_pass_t<double, M, LOGM>, st, nrows, false, in, nrows, n, rpp, out, tw);
 }
-
 template <int M, int LOGM>
-cudaError_t pass_eig(cudaStream_t st, const double* in, int nrows, int n, int rpp, const double* eig,
-                     double* out, const hpq::Cx<double>* tw) {
-    const int rb = hpq::DstCfg<M>::RB;
-    const size_t smem = smem_t<M>() + (size_t)rb * n * sizeof(double);
-    hpq::k_dst_pass_eig<double, M, LOGM, hpq::DstCfg<M>::RB><<<(nrows + rb - 1) / rb, 256, smem, st>>>(in, nrows, n, rpp, eig, out, tw);
-    return cudaGetLastError();
+cudaError_t pass_eig(cudaStream_t st, const double* in, int nx, int ny, double dx, double dy, double* out,
+                     const hpq::Cx<double>* tw) {
+    return launch<M>(k_pass_eig<M, LOGM>, st, nx, true, in, nx, ny, dx, dy, out, tw);
 }
-
 // The last x-pass writes a plain nx x ny plane (the caller's solution buffer): a slab view with
 // no guard cells, i.e. pitch nx and the guard offset removed from the base pointer.
 template <int M, int LOGM>
 cudaError_t pass_plane(cudaStream_t st, const double* in, int nrows, int n, int ny, double* out,
                        const hpq::Cx<double>* tw) {
-    const int rb = hpq::DstCfg<M>::RB;
-    const size_t smem = smem_t<M>();
     const int G = hpq::kGuardAlloc;
     double* base = out - ((ptrdiff_t)G * n + G);  // element (i, j) -> out[j * n + i]
-    hpq::k_dst_pass_field<double, M, LOGM, hpq::DstCfg<M>::RB><<<(nrows + rb - 1) / rb, 256, smem, st>>>(
-        in, nrows, n, ny, base, 0, n, 0, 0, 0, tw);
-    return cudaGetLastError();
+    return launch<M>(hpq::k_dst_pass_field<double, M, LOGM>, st, nrows, true, in, nrows, n, ny, base, (size_t)0, n, 0, 0, 0, tw);
 }
 
 int pow2_len(int n) {
@@ -167,19 +180,11 @@ extern "C" int hpq_poisson_dirichlet_noalloc(const double* f, double* u, int nx,
     // an error left pending by the caller's earlier work stays the caller's: nothing is launched
     // and it is not cleared
     if (cudaPeekAtLastError() != cudaSuccess) return HPQ_ERR_CUDA;
-    double* scratch = nullptr;
-    if (int r = scratch_for_current_device(&scratch)) return r;
+    double* work = nullptr;  // y-transformed intermediate, nx*ny
+    const hpq::Cx<double>* tw = nullptr;
+    if (int r = scratch_for_current_device(&work, &tw)) return r;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    double* work = scratch;                        // y-transformed intermediate, nx*ny
-    double* eig = scratch + kPlane;                // eigenvalues, nx*ny
-    auto* twx = reinterpret_cast<hpq::Cx<double>*>(scratch + 2 * kPlane);  // Mx/2 complex
-    auto* twy = twx + kTw / 2;                                              // My/2 complex
-    k_fill_eig<<<148, 256, 0, st>>>(eig, nx, ny, dx, dy);
-    if (cudaGetLastError() != cudaSuccess) return HPQ_ERR_CUDA;
-    k_fill_twiddles<<<4, 256, 0, st>>>(twx, Mx);
-    if (cudaGetLastError() != cudaSuccess) return HPQ_ERR_CUDA;
-    k_fill_twiddles<<<4, 256, 0, st>>>(twy, My);
-    if (cudaGetLastError() != cudaSuccess) return HPQ_ERR_CUDA;
+    const auto *twx = tw + tw_offset(Mx), *twy = tw + tw_offset(My);
     cudaError_t e = cudaSuccess;
     // x-pass of f -> u (transposed, u serves as the temporary); y-pass * eig * y-pass of u ->
     // work; x-pass of work -> u. No pass reads and writes the same buffer.
@@ -187,7 +192,7 @@ extern "C" int hpq_poisson_dirichlet_noalloc(const double* f, double* u, int nx,
     HPQ_NOALLOC_DISPATCH(Mx, CALL1)
 #undef CALL1
     if (e != cudaSuccess) return HPQ_ERR_CUDA;
-#define CALL2(M, L) pass_eig<M, L>(st, u, nx, ny, nx, eig, work, twy)
+#define CALL2(M, L) pass_eig<M, L>(st, u, nx, ny, dx, dy, work, twy)
     HPQ_NOALLOC_DISPATCH(My, CALL2)
 #undef CALL2
     if (e != cudaSuccess) return HPQ_ERR_CUDA;
