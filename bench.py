@@ -41,11 +41,10 @@ PUSH_BYTES = {8: 5 * 8 + 1 + 10 * 8, 4: 5 * 4 + 1 + 10 * 4}
 # the first smoothing
 MG_REALS_PER_POINT_VCYCLE = 4.0 / 3.0 * 9.0
 MG_REALS_PER_POINT_FIRST = 9.0
-# DRAM bytes (read 2 936 064 + write 0) of one k_mg_solve launch of the current kernel (two
-# coarse-level blocks) from ncu (blowout_255, FP64, one launch after 300, `--set full`,
-# profiles/k_mg_solve_blowout_255_fp64.md): the level-0 arrays stay in L2, so DRAM traffic is far
-# below the algorithmic bytes
-MG_NCU_DRAM_BYTES_FP64_255 = 2936064
+# DRAM bytes of one k_mg_cluster launch from ncu (255 x 255, FP64, three V-cycles,
+# profiles/k_mg_cluster_255_fp64.md): the hierarchy stays in shared memory during the solve, so DRAM
+# traffic is far below the algorithmic bytes
+MG_NCU_DRAM_BYTES_FP64_255 = 3330000
 
 
 def parse():
@@ -259,13 +258,13 @@ def run_ours(args):
         "e2e": {"value": e2e_value, "unit": "slices/s", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h},
         "gpu_launches": None,
-        "roofline": {"bound": "hbm", "kernel": "k_mg_solve", "achieved": mg_achieved, "peak": peak,
+        "roofline": {"bound": "hbm", "kernel": "k_mg_cluster" if max(nx, ny) <= 256 else "k_mg_solve", "achieved": mg_achieved, "peak": peak,
                      "unit": "GB/s", "frac": mg_achieved / peak, "peak_kind": peak_kind,
                      "traffic": (MG_NCU_DRAM_BYTES_FP64_255
                                  if (args.config == "blowout_255" and elem == 8) else None),
                      "bytes_per_launch": mg_bytes, "launch_ms": mg_launch_ms,
                      "vcycles_per_launch": vc,
-                     "note": "latency-bound: level-0 arrays live in L2; traffic from ncu, one cold launch"},
+                     "note": "latency-bound: the levels live in shared memory (k_mg_cluster) or L2; traffic from ncu, one cold launch"},
         "roofline_plasma_push": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                                  "frac": achieved / peak, "bytes_per_launch": push_bytes,
                                  "launch_ms": push_ms / max(push_n, 1)},

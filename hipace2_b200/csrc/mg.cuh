@@ -63,6 +63,17 @@ __device__ __forceinline__ R mg_diag_inv(const MGLev& L, int i, int j, R a, R fa
     if (CELL && (j == 0 || j == L.h - 1)) c0 -= R(2.) * facy;
     return R(1.) / c0;
 }
+// What rounding took from hi = -facx / diagonal (an error-free sum of the diagonal in units of facx,
+// one Newton step; hi = 0 outside the grid gives 0). A sweep that weights its neighbours with hi alone
+// solves an equation whose coefficient is off by up to 6e-8 * 4 / dx^2: in single precision 3e-3 of
+// chi = 1 at 2047^2, and as much of the fields. edge_x, edge_y: first or last cell (cell-centred).
+template <class R>
+__device__ __forceinline__ R mg_weight_low(bool edge_x, bool edge_y, R a, R facx, R ratio, R hi) {
+    const R wx = edge_x ? R(4) : R(2), wy = (edge_y ? R(4) : R(2)) * ratio, al = a / facx;
+    const R w = wx + wy, bw = w - wx, ew = (wx - (w - bw)) + (wy - bw);
+    const R d = w + al, bd = d - w, ed = (w - (d - bd)) + (al - bd);
+    return -(fma(hi, d, R(-1)) + hi * (ew + ed)) * hi;
+}
 template <class R, bool CELL>
 __device__ __forceinline__ R mg_gs_inv(const MGLev& L, int i, int j, R pim, R pip, R pjm, R pjp, R rhs, R c0_inv,
                                        R facx, R facy) {
@@ -1446,6 +1457,12 @@ __global__ void __launch_bounds__(256, 2) k_mg_solve(MGSolveArgs<R> P) {
     }
 }
 
+}  // namespace hpq
+
+#include "mgcl.cuh"
+
+namespace hpq {
+
 // ------------------------------------------------------------------------------------------
 template <class R>
 class Multigrid {
@@ -1537,6 +1554,115 @@ public:
         if (cell) HPQ_CUDA(cudaFuncSetAttribute(k_mg_bottom<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bottom_smem));
         else HPQ_CUDA(cudaFuncSetAttribute(k_mg_bottom<R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bottom_smem));
         if (cell) setup_persistent<true>(); else setup_persistent<false>();
+        if (coop_ok) { if (cell) setup_cluster<true>(); else setup_cluster<false>(); }
+    }
+
+    // cluster form (mgcl.cuh), for grids that fit it; cl64: single-precision slice arrays, FP64
+    // solve (tolerances below kRefineTol)
+    ClPlan<R> cl;
+    ClPlan<double> cl64;
+    unsigned long long* cl_slot = nullptr;  // ClArgs::slot
+    void* cl_coef = nullptr;                // ClArgs::coef
+
+    template <class IO, class RS, bool CELL>
+    void plan_cluster(ClPlan<RS>& pl) {
+        auto kern = k_mg_cluster<IO, RS, CELL>;
+        cudaFuncAttributes fa{};
+        HPQ_CUDA(cudaFuncGetAttributes(&fa, kern));
+        const size_t limit = 227 * 1024 - fa.sharedSizeBytes;
+        // a whole component in one block where it fits (63^2 in double): a sweep then ends with a
+        // block barrier (45 cycles) instead of a cluster barrier (500); else the largest cluster. A
+        // level runs in block 0 where its points there cost less than a cluster barrier, as far
+        // as the shared memory reaches.
+        struct Try { int cs, own; };
+        const Try tries[] = {{1, 1 << 30}, {16, 4225}, {16, 1100}, {16, 300}, {8, 4225}, {8, 1100}, {8, 300}};
+        for (const Try& t : tries) {
+            if (!ClPlan<RS>::layout(pl.a, pl.smem, lev, dx, dy, t.cs, t.own, coarse.ns_bottom) || pl.smem > limit) continue;
+            HPQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
+            HPQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            HPQ_CUDA(cudaFuncSetAttribute(k_mg_cluster_coef<IO, RS, CELL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
+            HPQ_CUDA(cudaFuncSetAttribute(k_mg_cluster_coef<IO, RS, CELL>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            cudaLaunchConfig_t cfg{};
+            cudaLaunchAttribute at[1];
+            cluster_config(cfg, at, pl.a.cs, pl.smem, nullptr);
+            int n = 0;
+            // (both components' clusters have to be resident: they exchange norms)
+            if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 2) { cudaGetLastError(); continue; }
+            pl.ok = true;
+            return;
+        }
+    }
+    static void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, int cs, size_t smem, cudaStream_t st) {
+        cfg.gridDim = dim3(2 * cs);
+        cfg.blockDim = dim3(kClThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim = {(unsigned)cs, 1, 1};
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+    }
+    template <bool CELL>
+    void setup_cluster() {
+        // HPQ_MG=tiles, or a variable that selects a form of the tile kernel, keeps the tile form
+        const char* e = getenv("HPQ_MG");
+        if (e && std::string(e) == "tiles") return;
+        for (const char* v : {"HPQ_MG_SPLIT", "HPQ_MG_T0", "HPQ_MG_L1", "HPQ_MG_TRACE", "HPQ_MG_WARP"})
+            if (getenv(v)) return;
+        plan_cluster<R, R, CELL>(cl);
+        if constexpr (std::is_same<R, float>::value) plan_cluster<float, double, CELL>(cl64);
+        const size_t bytes = std::max(cl.ok ? cl.a.cs * (size_t)cl.a.coef_elems * sizeof(R) : 0,
+                                      cl64.ok ? cl64.a.cs * (size_t)cl64.a.coef_elems * sizeof(double) : 0);
+        if (bytes) {
+            HPQ_CUDA(cudaMalloc(&cl_slot, 6 * kClMaxBlocks * sizeof(unsigned long long)));
+            HPQ_CUDA(cudaMalloc(&cl_coef, bytes));
+            HPQ_CUDA(cudaMemset(cl_coef, 0, bytes));
+        }
+    }
+    // single precision refines level 0 in FP64 only where the tolerance asks for it: an FP32 V-cycle
+    // reaches relative residuals well below kRefineTol on its own
+    bool refined(double tol_rel) const {
+        return std::is_same<R, float>::value && (refine_force >= 0 ? refine_force == 1 : tol_rel < kRefineTol);
+    }
+    ClView<R> cluster_view(const Slab<R>& S, int c0, int c1) const { return {{S.c(c0).p, S.c(c1).p}, S.pitch, kGuardAlloc}; }
+    template <class RS>
+    ClArgs<RS> cluster_args(const ClPlan<RS>& pl, Ctl* ctl) const {
+        ClArgs<RS> A = pl.a;
+        A.ctl = ctl;
+        A.slot = cl_slot;
+        A.coef = static_cast<RS*>(cl_coef);
+        return A;
+    }
+    template <class RS, bool CELL>
+    void launch_coef(cudaStream_t st, const Slab<R>& S, Ctl* ctl, const ClPlan<RS>& pl) {
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute at[1];
+        cluster_config(cfg, at, pl.a.cs, pl.smem, st);
+        cfg.gridDim = dim3(pl.a.cs);
+        HPQ_CUDA(cudaLaunchKernelEx(&cfg, k_mg_cluster_coef<R, RS, CELL>, cluster_args(pl, ctl), cluster_view(S, C_CHI, C_CHI)));
+        HPQ_LAUNCH_CHECK();
+    }
+    // The part of a solve that depends on chi alone, on stream `st`, ahead of solve_persistent(...,
+    // prepared = true) on the same slab; false: this grid has none
+    bool cluster_form(double tol_rel) const { return coop_ok && (refined(tol_rel) ? cl64.ok : cl.ok); }
+    void prepare(cudaStream_t st, const Slab<R>& S, Ctl* ctl, double tol_rel) {
+        if (refined(tol_rel)) {
+            if (cell) launch_coef<double, true>(st, S, ctl, cl64); else launch_coef<double, false>(st, S, ctl, cl64);
+        } else {
+            if (cell) launch_coef<R, true>(st, S, ctl, cl); else launch_coef<R, false>(st, S, ctl, cl);
+        }
+    }
+    template <class RS, bool CELL>
+    void launch_cluster(cudaStream_t st, const Slab<R>& S, Ctl* ctl, const ClPlan<RS>& pl, double tol_rel, double tol_abs,
+                        int maxiter, bool prepared) {
+        if (!prepared) launch_coef<RS, CELL>(st, S, ctl, pl);
+        ClArgs<RS> A = cluster_args(pl, ctl);
+        A.tol_rel = tol_rel; A.tol_abs = tol_abs; A.maxiter = maxiter;
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute at[1];
+        cluster_config(cfg, at, A.cs, pl.smem, st);
+        HPQ_CUDA(cudaLaunchKernelEx(&cfg, k_mg_cluster<R, RS, CELL>, A, cluster_view(S, C_BX, C_BY), cluster_view(S, C_SY, C_SX)));
+        HPQ_LAUNCH_CHECK();
     }
 
     // persistent solve: one cooperative launch with as many co-resident blocks as there are
@@ -1666,7 +1792,14 @@ public:
     }
 
     template <bool CELL>
-    void solve_persistent(cudaStream_t st, const Slab<R>& S, Ctl* ctl, double tol_rel, double tol_abs, int maxiter) {
+    void solve_persistent(cudaStream_t st, const Slab<R>& S, Ctl* ctl, double tol_rel, double tol_abs, int maxiter,
+                          bool prepared = false) {
+        const bool refine = refined(tol_rel);
+        if (refine ? cl64.ok : cl.ok) {
+            if (refine) launch_cluster<double, CELL>(st, S, ctl, cl64, tol_rel, tol_abs, maxiter, prepared);
+            else launch_cluster<R, CELL>(st, S, ctl, cl, tol_rel, tol_abs, maxiter, prepared);
+            return;
+        }
         MGSolveArgs<R> P{};
         P.nl = nl;
         P.sb = sb;
@@ -1686,9 +1819,7 @@ public:
         P.r32[0] = r32[0]; P.r32[1] = r32[1];
         P.trace = trace;
         P.split0 = split0 ? 1 : 0;
-        // single precision refines level 0 in FP64 only where the tolerance asks for it: an FP32
-        // V-cycle reaches relative residuals well below kRefineTol on its own
-        P.refine = std::is_same<R, float>::value && (refine_force >= 0 ? refine_force == 1 : tol_rel < kRefineTol);
+        P.refine = refine;
         // norms and barrier state; the timeout flag stays set until the step ends, so that after
         // a timeout the remaining solves of the step leave at their first barrier
         static_assert(offsetof(Ctl, mgp_bar_err) - offsetof(Ctl, mgp_rhsnorm) == 32, "Ctl layout");
@@ -1722,6 +1853,12 @@ public:
         coarse.garena = nullptr;
         if (trace) cudaFree(trace);
         trace = nullptr;
+        if (cl_slot) cudaFree(cl_slot);
+        if (cl_coef) cudaFree(cl_coef);
+        cl_slot = nullptr;
+        cl_coef = nullptr;
+        cl = ClPlan<R>{};
+        cl64 = ClPlan<double>{};
         for (int k = 0; k < 2; ++k) {
             if (x64[k]) cudaFree(x64[k]);
             if (r32[k]) cudaFree(r32[k]);

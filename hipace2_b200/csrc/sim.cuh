@@ -1484,18 +1484,19 @@ public:
         }
     }
 
-    void mg_solve() {
+    // prepared: Multigrid::prepare has run on this slice's chi
+    void mg_solve(bool prepared = false) {
         Scope sc(this, "multigrid");
-        if (mg.cell) mg_solve_t<true>(S); else mg_solve_t<false>(S);
+        if (mg.cell) mg_solve_t<true>(S, prepared); else mg_solve_t<false>(S, prepared);
     }
     // the multigrid reads Sy, Sx, chi and writes Bx, By of slab MS
     template <bool CELL>
-    void mg_solve_t(const Slab<R>& MS) { mg_run<CELL>(mg, MS); }
+    void mg_solve_t(const Slab<R>& MS, bool prepared = false) { mg_run<CELL>(mg, MS, prepared); }
     template <bool CELL, class MGT, class RS>
-    void mg_run(MGT& mg, const Slab<RS>& MS) {
+    void mg_run(MGT& mg, const Slab<RS>& MS, bool prepared = false) {
         if (mg.coop_ok) {
-            // the whole solve, iterations and decisions included, is one cooperative kernel
-            mg.template solve_persistent<CELL>(st, MS, ctl, cfg.mg_tol_rel, cfg.mg_tol_abs, cfg.mg_max_iters);
+            // the whole solve, iterations and decisions included, is one kernel
+            mg.template solve_persistent<CELL>(st, MS, ctl, cfg.mg_tol_rel, cfg.mg_tol_abs, cfg.mg_max_iters, prepared);
             return;
         }
         if (capturing) {
@@ -2095,10 +2096,18 @@ public:
                              cfg.do_beam_jx_jy_deposition ? S.c(C_JY).p : nullptr, S.c(C_JZ).p,
                              cfg.do_beam_jz_minus_rho ? S.c(C_RHOMJZ).p : nullptr);
         }
+        // the multigrid's coefficient hierarchy needs chi alone: beside the Poisson solves and the
+        // explicit deposit
+        const bool prepared = ex && mg.cluster_form(cfg.mg_tol_rel);
+        if (prepared) {
+            OnStream on(this, side_begin());
+            mg.prepare(st, S, ctl, cfg.mg_tol_rel);
+        }
         field_solve_psi_ez_bz();
         if (ex) {
             explicit_deposit();
-            mg_solve();
+            if (prepared) side_end();
+            mg_solve(prepared);
             if (sal_step && !capturing && salame_slice(cur_islice)) salame(cur_islice);
         } else {
             pc_loop();
