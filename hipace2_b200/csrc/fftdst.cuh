@@ -26,59 +26,6 @@ __device__ __forceinline__ Cx<R> cmul(const Cx<R>& v0, const Cx<R>& w) {
     return {v0.re * w.re - v0.im * w.im, v0.re * w.im + v0.im * w.re};
 }
 
-// In-place radix-2 DIT FFT of nfft rows of length M held in bit-reversed order. Pairs of
-// consecutive radix-2 stages (lengths 2h and 4h) are done by one thread on 4 elements (a
-// radix-4 step with the same operations as the two radix-2 stages), so a length-2^k transform
-// needs ceil(k/2) block barriers instead of k; stage sizes are compile-time, indices are shifts.
-template <class R, int M, int LOGM>
-__device__ __forceinline__ void fft_block(Cx<R>* z, int nfft, const Cx<R>* __restrict__ tw) {
-    static_assert((1 << LOGM) == M, "M = 2^LOGM");
-    int s = 0;  // stage length 2h with h = 2^s
-    if (LOGM & 1) {
-        for (int t = threadIdx.x; t < nfft * (M / 2); t += blockDim.x) {
-            const int f = t >> (LOGM - 1), b = t & (M / 2 - 1);
-            Cx<R>* zz = z + f * M;
-            const int i0 = 2 * b, i1 = i0 + 1;
-            const Cx<R> w = tw[0];
-            const Cx<R> u = zz[i0], v = cmul(zz[i1], w);
-            zz[i0] = {u.re + v.re, u.im + v.im};
-            zz[i1] = {u.re - v.re, u.im - v.im};
-        }
-        __syncthreads();
-        s = 1;
-    }
-#pragma unroll
-    for (int ss = LOGM & 1; ss < LOGM; ss += 2) {
-        s = ss;
-        const int h = 1 << s;
-        for (int t = threadIdx.x; t < nfft * (M / 4); t += blockDim.x) {
-            const int f = t >> (LOGM - 2), b = t & (M / 4 - 1);
-            const int grp = b >> s, pos = b & (h - 1);
-            Cx<R>* zz = z + f * M;
-            const int i0 = grp * 4 * h + pos, i1 = i0 + h, i2 = i0 + 2 * h, i3 = i0 + 3 * h;
-            const Cx<R> wa = tw[pos * (M / (2 * h))];
-            const Cx<R> wb0 = tw[pos * (M / (4 * h))], wb1 = tw[(pos + h) * (M / (4 * h))];
-            Cx<R> x0 = zz[i0], x1 = zz[i1], x2 = zz[i2], x3 = zz[i3];
-            // stage of length 2h: (i0, i1) and (i2, i3)
-            Cx<R> v = cmul(x1, wa);
-            x1 = {x0.re - v.re, x0.im - v.im};
-            x0 = {x0.re + v.re, x0.im + v.im};
-            v = cmul(x3, wa);
-            x3 = {x2.re - v.re, x2.im - v.im};
-            x2 = {x2.re + v.re, x2.im + v.im};
-            // stage of length 4h: (i0, i2) and (i1, i3)
-            v = cmul(x2, wb0);
-            zz[i2] = {x0.re - v.re, x0.im - v.im};
-            zz[i0] = {x0.re + v.re, x0.im + v.im};
-            v = cmul(x3, wb1);
-            zz[i3] = {x1.re - v.re, x1.im - v.im};
-            zz[i1] = {x1.re + v.re, x1.im + v.im};
-        }
-        __syncthreads();
-    }
-    (void)s;
-}
-
 // ------------------------------------------------------------------------------------------
 // The transform of a row pair: FFT of length M = 2(n+1) with 8 elements per thread in registers
 // (Stockham autosort: radix-8 passes, then one of radix 8, 4 or 2), so that M = 2048 passes
@@ -202,15 +149,15 @@ __device__ __forceinline__ void load_odd(Cx<R> (&v)[8], int t, int n, Get get) {
 }
 
 // The rows of a block written transposed: out[(plane n + e) rows_per_plane + row], through shared
-// memory so that the block's rows of one e are written together. v[q < 4] holds elements
+// memory so that the block's rows of one e are written together. v[q < NQ] holds elements
 // t + q M/8 - 1 of the pair f.
-template <class R, int M>
+template <class R, int M, int NQ = 4>
 __device__ __forceinline__ void store_transposed(const Cx<R> (&v)[8], Cx<R>* smem, int f, int t, int r0, int nrows, int n,
                                                  int rows_per_plane, R* __restrict__ out) {
     using C = DstCfg<M>;
     __syncthreads();
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < NQ; ++q) {
         const int j = t + q * (M / 8);
         // DST-I of the pair: row 0 is -Im / 2, row 1 is Re / 2
         smem[(size_t)j * C::F + f] = {v[q].im * R(-0.5), v[q].re * R(0.5)};
@@ -223,6 +170,24 @@ __device__ __forceinline__ void store_transposed(const Cx<R> (&v)[8], Cx<R>* sme
     const int pl = row / rows_per_plane, rr = row - pl * rows_per_plane;
     R* o = out + (size_t)pl * n * rows_per_plane + rr;
     for (int e = threadIdx.x / C::RB; e < n; e += C::NT / C::RB) o[(size_t)e * rows_per_plane] = s[(e + 1) * C::RB + r];
+}
+
+// The rows of a pair written to field component comp[k] (rows are (plane k, j) of length n)
+template <class R, int M, int NQ = 4>
+__device__ __forceinline__ void store_field(const Cx<R> (&v)[8], int t, int row0, int nrows, int n, int ny, R* base,
+                                            size_t cstride, int pitch, int c0, int c1, int c2) {
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const int row = row0 + r;
+        if (row >= nrows) continue;
+        const int k = row / ny, j = row - k * ny;
+        R* o = base + (size_t)(k == 0 ? c0 : (k == 1 ? c1 : c2)) * cstride + (size_t)(j + kGuardAlloc) * pitch + kGuardAlloc;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const int i = t + q * (M / 8);
+            if (i >= 1 && i <= n) o[i - 1] = r ? v[q].re * R(0.5) : v[q].im * R(-0.5);
+        }
+    }
 }
 
 // Pass over rows: DST-I of every row of length n, written transposed:
@@ -306,18 +271,7 @@ __global__ void __launch_bounds__(DstCfg<M>::NT, 1024 / DstCfg<M>::NT) k_dst_pas
     Cx<R> v[8];
     load_odd<R, M>(v, t, n, get);
     fft_regs<R, M, LOGM>(v, z + f * C::MP, t, tw);
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        const int row = row0 + r;
-        if (row >= nrows) continue;
-        const int k = row / ny, j = row - k * ny;
-        R* o = base + (size_t)(k == 0 ? c0 : (k == 1 ? c1 : c2)) * cstride + (size_t)(j + kGuardAlloc) * pitch + kGuardAlloc;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int i = t + q * (M / 8);
-            if (i >= 1) o[i - 1] = r ? v[q].re * R(0.5) : v[q].im * R(-0.5);
-        }
-    }
+    store_field<R, M>(v, t, row0, nrows, n, ny, base, cstride, pitch, c0, c1, c2);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -325,142 +279,109 @@ __global__ void __launch_bounds__(DstCfg<M>::NT, 1024 / DstCfg<M>::NT) k_dst_pas
 // computation of the discrete Fourier transform", 1970). With d_m = exp(-i pi m^2 / M), the DFT of
 // the odd extension z (length M = 2(n+1), not a power of two) is
 //   Z[k] = d_k sum_j (z_j d_j) conj(d_{k-j}),
-// a circular convolution of length L (a power of two >= 2M - 1) done with two radix-2 FFTs of
-// length L: the forward one decimated in frequency (natural order in, bit-reversed out), the
-// product with B = FFT(conj(d)) held in bit-reversed order, and the inverse through
-// conj(FFT(conj(.))) decimated in time (bit-reversed in, natural out). No permutation pass.
+// a circular convolution of length L (a power of two >= 2M - 1) done with two FFTs of length L: the
+// forward one, the product with B = FFT(conj(d)), and the inverse through conj(FFT(conj(.))). The FFTs
+// are the register FFT above; z fills less than half of L, and Z is needed in less than a quarter.
 // ------------------------------------------------------------------------------------------
 template <class R>
 struct BluAxis {
     const Cx<R>* d;    // chirp d_m, m < M
-    const Cx<R>* B;    // FFT_L of the chirp filter conj(d_|m|), bit-reversed order
+    const Cx<R>* B;    // FFT_L of the chirp filter conj(d_|m|), divided by L
     const Cx<R>* tw;   // exp(-2 pi i t / L), t < L/2
     int M;
 };
 
-// In-place radix-2 DIF FFT of nfft rows of length L (natural order in, bit-reversed order out)
-template <class R, int L, int LOGL>
-__device__ __forceinline__ void fft_block_dif(Cx<R>* z, int nfft, const Cx<R>* __restrict__ tw) {
-#pragma unroll 1
-    for (int s = LOGL - 1; s >= 0; --s) {
-        const int h = 1 << s;
-        for (int t = threadIdx.x; t < nfft * (L / 2); t += blockDim.x) {
-            const int f = t >> (LOGL - 1), b = t & (L / 2 - 1);
-            const int grp = b >> s, pos = b & (h - 1);
-            Cx<R>* zz = z + f * L;
-            const int i0 = grp * 2 * h + pos, i1 = i0 + h;
-            const Cx<R> u = zz[i0], v = zz[i1];
-            zz[i0] = {u.re + v.re, u.im + v.im};
-            zz[i1] = cmul(Cx<R>{u.re - v.re, u.im - v.im}, tw[pos << (LOGL - 1 - s)]);
-        }
-        __syncthreads();
-    }
-}
-
-// DFT of the odd extensions of nfft row pairs into z (row f: complex z[f * L + k] such that
-// blu_val reads the DST-I); get(r, e) returns element e of block row r
+// DST-I of one row pair by the L/8 threads t: on return v[q], q < 2, holds {row 1, -row 0} times 2 at
+// element t + q L/8 - 1, as the power-of-two transform leaves it
 template <class R, int L, int LOGL, class Get>
-__device__ __forceinline__ void blu_forward(Cx<R>* z, int nfft, int n, const BluAxis<R>& A, Get get) {
+__device__ __forceinline__ void blu_rows(Cx<R> (&v)[8], Cx<R>* z, int t, int n, const BluAxis<R>& A, Get get) {
     const int M = A.M;
-    for (int t = threadIdx.x; t < nfft * L; t += blockDim.x) {
-        const int f = t >> LOGL, j = t & (L - 1);
-        Cx<R> v{R(0), R(0)};
-        if (j < M) {
-            R re = 0, im = 0;
-            if (j >= 1 && j <= n) { re = get(2 * f, j - 1); im = get(2 * f + 1, j - 1); }
-            else if (j >= n + 2) { re = -get(2 * f, M - j - 1); im = -get(2 * f + 1, M - j - 1); }
-            v = cmul(Cx<R>{re, im}, A.d[j]);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int j = t + q * (L / 8);
+        v[q] = {R(0), R(0)};
+        if (q < 4 && j >= 1 && j < M && j != n + 1) {
+            const bool up = j <= n;
+            const int e = up ? j - 1 : M - j - 1;
+            const R sg = up ? R(1) : R(-1);
+            v[q] = cmul(Cx<R>{sg * get(0, e), sg * get(1, e)}, A.d[j]);
         }
-        z[t] = v;
+    }
+    const Cx<R>* tw = A.tw;
+    fft_regs<R, L, LOGL>(v, z, t, tw);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const Cx<R> p = cmul(v[q], A.B[t + q * (L / 8)]);
+        v[q] = {p.re, -p.im};
+    }
+    asm volatile("" : "+l"(tw));  // (read again rather than kept)
+    fft_regs<R, L, LOGL>(v, z, t, tw);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int k = t + q * (L / 8);
+        if (k < M) v[q] = cmul(Cx<R>{v[q].re, -v[q].im}, A.d[k]);
+    }
+}
+
+template <class R, int L, int LOGL>
+__global__ void __launch_bounds__(DstCfg<L>::NT, 1024 / DstCfg<L>::NT) k_dstb_pass_t(const R* __restrict__ in, int nrows,
+                                                                                     int n, int rows_per_plane,
+                                                                                     R* __restrict__ out, BluAxis<R> A) {
+    HPQ_PDL_ENTRY();
+    using C = DstCfg<L>;
+    extern __shared__ __align__(16) unsigned char dst_smem[];
+    Cx<R>* z = reinterpret_cast<Cx<R>*>(dst_smem);
+    const int f = threadIdx.x / C::T, t = threadIdx.x % C::T, r0 = blockIdx.x * C::RB, row0 = r0 + 2 * f;
+    auto get = [&](int r, int e) -> R { return row0 + r < nrows ? in[(size_t)(row0 + r) * n + e] : R(0); };
+    Cx<R> v[8];
+    blu_rows<R, L, LOGL>(v, z + f * C::MP, t, n, A, get);
+    store_transposed<R, L, 2>(v, z, f, t, r0, nrows, n, rows_per_plane, out);
+}
+
+template <class R, int L, int LOGL>
+__global__ void __launch_bounds__(DstCfg<L>::NT, 1024 / DstCfg<L>::NT) k_dstb_pass_eig(const R* __restrict__ in, int nrows,
+                                                                                       int n, int rows_per_plane,
+                                                                                       const R* __restrict__ eig,
+                                                                                       R* __restrict__ out, BluAxis<R> A) {
+    HPQ_PDL_ENTRY();
+    using C = DstCfg<L>;
+    extern __shared__ __align__(16) unsigned char dst_smem[];
+    Cx<R>* z = reinterpret_cast<Cx<R>*>(dst_smem);
+    const int f = threadIdx.x / C::T, t = threadIdx.x % C::T, r0 = blockIdx.x * C::RB, row0 = r0 + 2 * f;
+    auto get = [&](int r, int e) -> R { return row0 + r < nrows ? in[(size_t)(row0 + r) * n + e] : R(0); };
+    Cx<R> v[8];
+    Cx<R>* zf = z + f * C::MP;
+    blu_rows<R, L, LOGL>(v, zf, t, n, A, get);
+    const int i0 = row0 % rows_per_plane, i1 = (row0 + 1) % rows_per_plane;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int j = t + q * (L / 8);
+        if (j >= 1 && j <= n) {
+            const R* eg = eig + (size_t)(j - 1) * rows_per_plane;
+            zf[j - 1] = {row0 < nrows ? v[q].im * R(-0.5) * eg[i0] : R(0), row0 + 1 < nrows ? v[q].re * R(0.5) * eg[i1] : R(0)};
+        }
     }
     __syncthreads();
-    fft_block_dif<R, L, LOGL>(z, nfft, A.tw);
-    for (int t = threadIdx.x; t < nfft * L; t += blockDim.x) {
-        const Cx<R> p = cmul(z[t], A.B[t & (L - 1)]);
-        z[t] = {p.re, -p.im};
-    }
-    __syncthreads();
-    fft_block<R, L, LOGL>(z, nfft, A.tw);
+    auto get2 = [&](int r, int e) -> R { return r ? zf[e].im : zf[e].re; };
+    blu_rows<R, L, LOGL>(v, zf, t, n, A, get2);
+    store_transposed<R, L, 2>(v, z, f, t, r0, nrows, n, rows_per_plane, out);
 }
 
-// DST-I value of element e of block row r: Z[k] = d_k conj(y[k]) / L at k = e + 1
-template <class R, int L>
-__device__ __forceinline__ R blu_val(const Cx<R>* z, const BluAxis<R>& A, int r, int e) {
-    const Cx<R> y = z[(r >> 1) * L + e + 1];
-    const Cx<R> zk = cmul(Cx<R>{y.re, -y.im}, A.d[e + 1]);
-    return (r & 1) ? zk.re * (R(0.5) / R(L)) : -zk.im * (R(0.5) / R(L));
-}
-
-template <class R, int L, int LOGL, int RB>
-__global__ void __launch_bounds__(256) k_dstb_pass_t(const R* __restrict__ in, int nrows, int n, int rows_per_plane,
-                                                     R* __restrict__ out, BluAxis<R> A) {
+template <class R, int L, int LOGL>
+__global__ void __launch_bounds__(DstCfg<L>::NT, 1024 / DstCfg<L>::NT)
+    k_dstb_pass_field(const R* __restrict__ in, int nrows, int n, int ny, R* base, size_t cstride, int pitch, int c0, int c1,
+                      int c2, BluAxis<R> A) {
     HPQ_PDL_ENTRY();
-    extern __shared__ unsigned char smem_raw[];
-    Cx<R>* z = reinterpret_cast<Cx<R>*>(smem_raw);
-    const int r0 = blockIdx.x * RB;
-    auto get = [&](int r, int e) -> R { const int row = r0 + r; return row < nrows ? in[(size_t)row * n + e] : R(0); };
-    blu_forward<R, L, LOGL>(z, RB / 2, n, A, get);
-    for (int t = threadIdx.x; t < RB * n; t += blockDim.x) {
-        const int r = t % RB, e = t / RB;
-        const int row = r0 + r;
-        if (row >= nrows) continue;
-        const int pl = row / rows_per_plane, rr = row - pl * rows_per_plane;
-        out[((size_t)pl * n + e) * rows_per_plane + rr] = blu_val<R, L>(z, A, r, e);
-    }
+    using C = DstCfg<L>;
+    extern __shared__ __align__(16) unsigned char dst_smem[];
+    Cx<R>* z = reinterpret_cast<Cx<R>*>(dst_smem);
+    const int f = threadIdx.x / C::T, t = threadIdx.x % C::T, row0 = blockIdx.x * C::RB + 2 * f;
+    auto get = [&](int r, int e) -> R { return row0 + r < nrows ? in[(size_t)(row0 + r) * n + e] : R(0); };
+    Cx<R> v[8];
+    blu_rows<R, L, LOGL>(v, z + f * C::MP, t, n, A, get);
+    store_field<R, L, 2>(v, t, row0, nrows, n, ny, base, cstride, pitch, c0, c1, c2);
 }
-
-template <class R, int L, int LOGL, int RB>
-__global__ void __launch_bounds__(256) k_dstb_pass_eig(const R* __restrict__ in, int nrows, int n, int rows_per_plane,
-                                                       const R* __restrict__ eig, R* __restrict__ out, BluAxis<R> A) {
-    HPQ_PDL_ENTRY();
-    extern __shared__ unsigned char smem_raw[];
-    Cx<R>* z = reinterpret_cast<Cx<R>*>(smem_raw);
-    R* tmp = reinterpret_cast<R*>(z + (RB / 2) * L);
-    const int r0 = blockIdx.x * RB;
-    auto get = [&](int r, int e) -> R { const int row = r0 + r; return row < nrows ? in[(size_t)row * n + e] : R(0); };
-    blu_forward<R, L, LOGL>(z, RB / 2, n, A, get);
-    for (int t = threadIdx.x; t < RB * n; t += blockDim.x) {
-        const int r = t / n, e = t - r * n;
-        const int row = r0 + r;
-        const int i = row % rows_per_plane;
-        tmp[t] = row < nrows ? blu_val<R, L>(z, A, r, e) * eig[(size_t)e * rows_per_plane + i] : R(0);
-    }
-    __syncthreads();
-    auto get2 = [&](int r, int e) -> R { return tmp[r * n + e]; };
-    blu_forward<R, L, LOGL>(z, RB / 2, n, A, get2);
-    for (int t = threadIdx.x; t < RB * n; t += blockDim.x) {
-        const int r = t % RB, e = t / RB;
-        const int row = r0 + r;
-        if (row >= nrows) continue;
-        const int pl = row / rows_per_plane, rr = row - pl * rows_per_plane;
-        out[((size_t)pl * n + e) * rows_per_plane + rr] = blu_val<R, L>(z, A, r, e);
-    }
-}
-
-template <class R, int L, int LOGL, int RB>
-__global__ void __launch_bounds__(256) k_dstb_pass_field(const R* __restrict__ in, int nrows, int n, int ny, R* base,
-                                                         size_t cstride, int pitch, int c0, int c1, int c2, BluAxis<R> A) {
-    HPQ_PDL_ENTRY();
-    extern __shared__ unsigned char smem_raw[];
-    Cx<R>* z = reinterpret_cast<Cx<R>*>(smem_raw);
-    const int r0 = blockIdx.x * RB;
-    auto get = [&](int r, int e) -> R { const int row = r0 + r; return row < nrows ? in[(size_t)row * n + e] : R(0); };
-    blu_forward<R, L, LOGL>(z, RB / 2, n, A, get);
-    for (int t = threadIdx.x; t < RB * n; t += blockDim.x) {
-        const int r = t / n, e = t - r * n;
-        const int row = r0 + r;
-        if (row >= nrows) continue;
-        const int k = row / ny, j = row - k * ny;
-        const int comp = k == 0 ? c0 : (k == 1 ? c1 : c2);
-        base[(size_t)comp * cstride + (size_t)(j + kGuardAlloc) * pitch + (e + kGuardAlloc)] = blu_val<R, L>(z, A, r, e);
-    }
-}
-
-// rows per block of a Bluestein pass: the L-point complex rows of the row pairs must fit
-template <class R, int L>
-struct BluCfg {
-    static constexpr int RB = (size_t)2 * L * sizeof(Cx<R>) <= 96 * 1024 ? 4 : 2;
-};
 
 template <class R>
 class FastDST {
@@ -523,7 +444,7 @@ public:
                 }
         std::vector<Cx<R>> hd(M), hB(L);
         for (int m = 0; m < M; ++m) hd[m] = {(R)dre[m], (R)dim[m]};
-        for (int q = 0; q < L; ++q) hB[q] = {(R)br[rev(q)], (R)bi[rev(q)]};  // bit-reversed order
+        for (int q = 0; q < L; ++q) hB[q] = {(R)(br[q] / L), (R)(bi[q] / L)};
         BluAxis<R> A{};
         Cx<R>*d = nullptr, *B = nullptr;
         HPQ_CUDA(cudaMalloc(&d, M * sizeof(Cx<R>)));
@@ -576,32 +497,28 @@ public:
     }
     template <int L, int LOGL>
     static void set_attrs_blu() {
-        constexpr int RB = BluCfg<R, L>::RB;
-        const int big = 220 * 1024;
-        HPQ_CUDA(cudaFuncSetAttribute(k_dstb_pass_t<R, L, LOGL, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-        HPQ_CUDA(cudaFuncSetAttribute(k_dstb_pass_eig<R, L, LOGL, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-        HPQ_CUDA(cudaFuncSetAttribute(k_dstb_pass_field<R, L, LOGL, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+        const int smem = (int)DstCfg<L>::template smem<R>();
+        HPQ_CUDA(cudaFuncSetAttribute(k_dstb_pass_t<R, L, LOGL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        HPQ_CUDA(cudaFuncSetAttribute(k_dstb_pass_eig<R, L, LOGL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        HPQ_CUDA(cudaFuncSetAttribute(k_dstb_pass_field<R, L, LOGL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     }
-    template <int L>
-    static size_t smem_blu() { return (size_t)(BluCfg<R, L>::RB / 2) * L * sizeof(Cx<R>); }
     template <int L, int LOGL>
     void bpass_t(cudaStream_t st, const R* in, int nrows, int n, int rpp, R* out, const BluAxis<R>& A) {
-        constexpr int RB = BluCfg<R, L>::RB;
-        hpq_launch(k_dstb_pass_t<R, L, LOGL, RB>, dim3((nrows + RB - 1) / RB), dim3(256), smem_blu<L>(), st, in, nrows, n, rpp, out, A);
+        using C = DstCfg<L>;
+        hpq_launch(k_dstb_pass_t<R, L, LOGL>, dst_grid<L>(nrows), dim3(C::NT), C::template smem<R>(), st, in, nrows, n, rpp, out, A);
         HPQ_LAUNCH_CHECK();
     }
     template <int L, int LOGL>
     void bpass_eig(cudaStream_t st, const R* in, int nrows, int n, int rpp, const R* eig, R* out, const BluAxis<R>& A) {
-        constexpr int RB = BluCfg<R, L>::RB;
-        hpq_launch(k_dstb_pass_eig<R, L, LOGL, RB>, dim3((nrows + RB - 1) / RB), dim3(256),
-                   smem_blu<L>() + (size_t)RB * n * sizeof(R), st, in, nrows, n, rpp, eig, out, A);
+        using C = DstCfg<L>;
+        hpq_launch(k_dstb_pass_eig<R, L, LOGL>, dst_grid<L>(nrows), dim3(C::NT), C::template smem<R>(), st, in, nrows, n, rpp, eig, out, A);
         HPQ_LAUNCH_CHECK();
     }
     template <int L, int LOGL>
     void bpass_field(cudaStream_t st, const R* in, int nrows, int n, R* base, size_t cs, int pitch, const int* comps,
                      int nrhs, const BluAxis<R>& A) {
-        constexpr int RB = BluCfg<R, L>::RB;
-        hpq_launch(k_dstb_pass_field<R, L, LOGL, RB>, dim3((nrows + RB - 1) / RB), dim3(256), smem_blu<L>(), st,
+        using C = DstCfg<L>;
+        hpq_launch(k_dstb_pass_field<R, L, LOGL>, dst_grid<L>(nrows), dim3(C::NT), C::template smem<R>(), st,
                    in, nrows, n, ny, base, cs, pitch, comps[0], nrhs > 1 ? comps[1] : comps[0],
                    nrhs > 2 ? comps[2] : comps[0], A);
         HPQ_LAUNCH_CHECK();

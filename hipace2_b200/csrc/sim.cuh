@@ -529,22 +529,17 @@ public:
         HPQ_CUDA(cudaMemset(ctl, 0, sizeof(Ctl)));
         HPQ_CUDA(cudaMallocHost(&ctl_h, sizeof(Ctl)));
         std::memset(ctl_h, 0, sizeof(Ctl));
-        // Poisson form: single precision uses the radix-2 FP32 FFT on 2^k - 1 grids (at 255^2 as
-        // fast as the tensor-core GEMMs, 3438 vs 3429 slices/s, with 2.5x less error in Ez: 5.2e-4
-        // vs 1.3e-3 of FP64 in the blowout; at 2047^2 faster, 266 vs 249; at 1023^2 4 % slower,
-        // 582 vs 608) and the tensor-core sine GEMMs (TF32x3) on other grids up to 1023^2;
+        // Poisson form: the FFT on 2^k - 1 grids, and in double precision the Bluestein FFT on all
+        // others (whole steps on a B200 against the SIMT sine GEMMs: the 64^2 predictor-corrector
+        // linear wake 255 vs 337 us per slice, the three solves of 384 x 320 115 vs 345 us; the GEMMs,
+        // O(n^3), were not faster anywhere from 48 to 1200). Single precision takes the Bluestein FFT
+        // below 128 (transform length 512; 64^2 97 vs 109 us per slice) and the tensor-core sine GEMMs
+        // (TF32x3) above, up to 1023^2 (256^2 176 vs 197, 600^2 1340 vs 1713).
         // HPQ_DST=tc / tc_bf16 (BF16x3 tensor-core GEMMs) / fft / gemm (SIMT sine GEMMs on every
-        // grid, cross-checks) forces a form;
-        // double precision uses the radix-2 FFT on 2^k - 1 grids, the SIMT sine GEMMs on other
-        // grids up to 1024 (measured whole steps on a B200 against the Bluestein FFT: equal or
-        // faster from 48 to 1000, e.g. 13.8 vs 20.0 ms at 128^2 x 40 slices, 20.9 vs 29.0 at 256^2,
-        // 102.6 vs 110.2 at 600^2 x 16, the linear-wake predictor-corrector case at 64^2 3053 vs
-        // 1912 slices/s; up to 7 % slower on explicit decks below 128) and the Bluestein FFT beyond
+        // grid, cross-checks) forces a form
         const char* env = getenv("HPQ_DST");
         std::string dmode = env ? env : "";
-        if (dmode.empty() && std::is_same<R, float>::value && FastDST<R>::radix2(nx, ny)) dmode = "fft";
-        if (dmode.empty() && std::is_same<R, double>::value && !FastDST<R>::radix2(nx, ny) && std::max(nx, ny) <= 1024)
-            dmode = "gemm";
+        if (dmode.empty() && std::is_same<R, float>::value && (FastDST<R>::radix2(nx, ny) || std::max(nx, ny) < 128)) dmode = "fft";
         if (dmode == "gemm") { dst.set_mode(false); pc_dst.set_mode(false); if (sal_dst.nx) sal_dst.set_mode(false); }
         else if (dmode != "fft" && std::is_same<R, float>::value) {
             const bool bf16 = dmode == "tc_bf16";
