@@ -57,11 +57,15 @@ __device__ __forceinline__ R mg_lap(const MGLev& L, int i, int j, R pc, R pim, R
 // diagonal, which depends only on the coefficient and the position, is computed once per point
 // and reused by every colour sweep.
 template <class R, bool CELL>
-__device__ __forceinline__ R mg_diag_inv(const MGLev& L, int i, int j, R a, R facx, R facy) {
+__device__ __forceinline__ R mg_diag(const MGLev& L, int i, int j, R a, R facx, R facy) {
     R c0 = -(a + R(2.) * (facx + facy));
     if (CELL && (i == 0 || i == L.w - 1)) c0 -= R(2.) * facx;
     if (CELL && (j == 0 || j == L.h - 1)) c0 -= R(2.) * facy;
-    return R(1.) / c0;
+    return c0;
+}
+template <class R, bool CELL>
+__device__ __forceinline__ R mg_diag_inv(const MGLev& L, int i, int j, R a, R facx, R facy) {
+    return R(1.) / mg_diag<R, CELL>(L, i, j, a, facx, facy);
 }
 // What rounding took from hi = -facx / diagonal (an error-free sum of the diagonal in units of facx,
 // one Newton step; hi = 0 outside the grid gives 0). A sweep that weights its neighbours with hi alone
@@ -222,166 +226,197 @@ __device__ __forceinline__ R mg_interp1f(const C& crse, int i, int j) {
     return crse(ic, jc);
 }
 
+// The loaded region of a T x T tile (256 threads): NSW halo cells, two more where the residual is
+// formed on the tile and a ring around it. A thread owns the column pair k of RT consecutive rows.
+template <int T, int NSW, bool RES>
+struct SmoothCfg {
+    static constexpr int H = RES ? NSW + 2 : NSW;
+    static constexpr int E = T + 2 * H;
+    static constexpr int KP = E / 2;            // column pairs
+    static constexpr int RS = 2 * KP + 2;       // a row in shared memory: even columns, 0, 0, odd columns
+    static constexpr int RT = (E + 256 / KP - 1) / (256 / KP);
+    // rows above and below of zeros, and the rows that the last strip has beyond E (read, never written)
+    static constexpr int PLANE = ((E + RT - 1) / RT * RT + 2) * RS;
+};
 template <int T, int NSW>
 struct SmoothSmem {
-    static constexpr int H = NSW + 2;  // exact residual on the tile and its ring after NSW sweeps
-    static constexpr int E = T + 2 * H;
-    static constexpr int Q = T + 2;
-    static constexpr int EC = E / 2 + 3;  // coarse points under the loaded region (interpolation)
-    // phi (2), rhs (2), coefficient, 1/diagonal, then the coarse correction (2, read before the
-    // sweeps); the residual (2 Q^2) reuses the 1/diagonal and coarse planes after the sweeps
-    static constexpr int TAIL = (E * E + 2 * EC * EC > 2 * Q * Q) ? E * E + 2 * EC * EC : 2 * Q * Q;
     template <class R>
-    static constexpr size_t bytes() { return (size_t)(5 * E * E + TAIL) * sizeof(R); }
+    static constexpr size_t bytes() { return (size_t)2 * SmoothCfg<T, NSW, true>::PLANE * sizeof(R); }
 };
 
 // One T x T tile (tile coordinates bx, by) of the fused smoother. `swap` selects in2/out2 for
 // in/out. The tile's residual and |rhs| max norms are folded into the caller's bmax / brhs.
+//
+// Both components of a point pair sit in one thread's registers, by colour e = (i + j) & 1: a sweep
+// updates u[.][.][e] from u[.][.][1 - e] of the thread's own rows and pair, and reads only the
+// pair's outer neighbour and the rows beyond its strip from shared memory (rows with even columns
+// first, so that threads read consecutive words). Shared-memory traffic bounds the sweeps: the form
+// that kept rhs, diagonal and all neighbours there, two words apart, moved 4 times as much
+// (1023^2 in double: 58 and 52 us for the two level-0 passes of a V-cycle; the whole solve of a slice took
+// 677 us and takes 479, in single precision 508 and 437; 2047^2 single 1415 and 1352). A colour sweep reads
+// the other colour only, so the guess is loaded for colour 1 alone (the first sweep replaces
+// colour 0), and after the last sweep the residual of colour 1 is zero up to rounding: the norm
+// and the restriction take colour 0, whose residual is the diagonal times the change a further
+// sweep would make.
 template <class R, bool CELL, int T, int INIT, bool RES, bool RESTR, int NORM, int NSW>
 __device__ __forceinline__ void mg_smooth_tile(const SmoothArgs<R>& A, int bx, int by, bool swap,
                                                unsigned char* smem_raw, double& bmax, double& brhs) {
-    using SM = SmoothSmem<T, NSW>;
-    constexpr int H = SM::H;
-    constexpr int E = SM::E;
-    constexpr int Q = SM::Q;  // residual tile with its ring
-    constexpr int NT = 256;   // threads of every smoother launch
-    R (*sp)[E * E] = reinterpret_cast<R (*)[E * E]>(smem_raw);                 // phi, 2 comps
-    R (*srh)[E * E] = reinterpret_cast<R (*)[E * E]>(smem_raw + 2 * E * E * sizeof(R));  // rhs
-    R* sa = reinterpret_cast<R*>(smem_raw + 4 * E * E * sizeof(R));             // coefficient
-    R* sinv = reinterpret_cast<R*>(smem_raw + 5 * E * E * sizeof(R));           // 1 / diagonal
-    constexpr int EC = SM::EC;
-    R (*sc)[EC * EC] = reinterpret_cast<R (*)[EC * EC]>(smem_raw + 6 * E * E * sizeof(R));  // coarse (set-up only)
-    // residual: written after the last sweep's barrier, over the 1/diagonal and coarse planes
-    R (*sr)[Q * Q] = reinterpret_cast<R (*)[Q * Q]>(smem_raw + 5 * E * E * sizeof(R));
+    using C = SmoothCfg<T, NSW, RES>;
+    constexpr int H = C::H, E = C::E, KP = C::KP, RS = C::RS, RT = C::RT;
+    static_assert(H % 2 == 0 && T % 2 == 0, "colours of the tile are those of the grid");
+    R* sm = reinterpret_cast<R*>(smem_raw);
     const MGLev& L = A.L;
     const int t0i = L.vlo + bx * T, t0j = L.vlo + by * T;
     const int ti0 = t0i - H, tj0 = t0j - H;
     const MV<R> vin = swap ? A.in2 : A.in;
     const MV<R> vout = swap ? A.out2 : A.out;
+    const int g = (int)threadIdx.x / KP, k = (int)threadIdx.x - g * KP, r0 = g * RT, par = r0 & 1;
+    // words of the column of colour 0 in rows q even, of colour 0 in rows q odd, and of the outer neighbours
+    const int own0 = par ? KP + 2 + k : k, own1 = par ? k : KP + 2 + k;
+    const int out0 = par ? k + 1 : KP + 1 + k, out1 = par ? KP + 1 + k : k + 1;
+    const bool act = r0 < E;
+    const R fx = A.facx, fy = A.facy, ratio = fy / fx;
+    // solution, rhs / diagonal, -facx / diagonal and its low part, diagonal of colour 0. (The low part is
+    // taken in single precision wherever a solution is swept, in every sweep, so that a pass of 8 sweeps and two
+    // of 4 stay the same bit for bit; adding its share to rhs / diagonal in the first sweep alone saved 6 of
+    // 437 us per slice at 1023^2. A level that starts from zero holds a correction, to which an error
+    // of its size does not matter.)
+    constexpr bool LOW = std::is_same<R, float>::value && INIT != MG_INIT_ZERO;
+    R u[2][RT][2], rv[2][RT][2], cx[RT][2], low[RT][2], c0[RT];
+    auto column = [&](int q, int e) { return 2 * k + ((e ^ (par + q)) & 1); };
+#pragma unroll
+    for (int q = 0; q < RT; ++q)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int li = column(q, e), lj = r0 + q, i = ti0 + li, j = tj0 + lj;
+            const bool v = act && lj < E && i >= L.vlo && i <= L.vhi_i && j >= L.vlo && j <= L.vhi_j;
+            const R a = v ? A.acf(i, j, 0) : R(0);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                rv[c][q][e] = v ? A.rhs(i, j, c) : R(0);
+                u[c][q][e] = R(0);
+                if (e == 1 && v && (INIT == MG_INIT_VIEW || INIT == MG_INIT_INTERP)) u[c][q][e] = vin(i, j, c);
+            }
+            if (e == 1 && v && (INIT == MG_INIT_INTERP || INIT == MG_INIT_INTERP0)) {
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+                    u[c][q][e] += mg_interp1f<R, CELL>([&](int ic, int jc) { return A.crse_in(ic, jc, c); }, i, j);
+            }
+            const R d = mg_diag<R, CELL>(L, i, j, a, fx, fy), inv = v ? R(1) / d : R(0);
+            if (e == 0) c0[q] = v ? d : R(0);
+            cx[q][e] = -fx * inv;
+            low[q][e] = LOW ? mg_weight_low<R>(CELL && (i == 0 || i == L.w - 1), CELL && (j == 0 || j == L.h - 1), a, fx, ratio, cx[q][e]) : R(0);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                if (NORM == MG_NORM_FIRST && li >= H && li < H + T && lj >= H && lj < H + T)
+                    brhs = fmax(brhs, fabs((double)rv[c][q][e]));
+                rv[c][q][e] *= inv;
+            }
+        }
     __syncthreads();  // shared memory of the previous tile of this block
-    // every global read of the tile is an asynchronous copy issued here, all in flight together
-    // (cells outside the valid box are zero-filled)
-    const int ci0 = (ti0 >> 1) - 1, cj0 = (tj0 >> 1) - 1;  // coarse origin of the interpolation
-#pragma unroll
-    for (int e0 = 0; e0 < E * E; e0 += NT) {
-        const int e = e0 + threadIdx.x;
-        if (e >= E * E) break;
-        const int i = ti0 + e % E, j = tj0 + e / E;
-        const bool v = i >= L.vlo && i <= L.vhi_i && j >= L.vlo && j <= L.vhi_j;
-        cp_async_el<R>(&sa[e], v ? &A.acf(i, j, 0) : A.acf.p[0], v);
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-            cp_async_el<R>(&srh[c][e], v ? &A.rhs(i, j, c) : A.rhs.p[c], v);
-            if (INIT == MG_INIT_ZERO || INIT == MG_INIT_INTERP0) sp[c][e] = R(0);
-            else cp_async_el<R>(&sp[c][e], v ? &vin(i, j, c) : vin.p[c], v);
-        }
+    for (int t = threadIdx.x; t < 2 * RS; t += 256) {
+        sm[t < RS ? t : (E + 1) * RS + t - RS] = R(0);
+        sm[C::PLANE + (t < RS ? t : (E + 1) * RS + t - RS)] = R(0);
     }
-    if (INIT == MG_INIT_INTERP || INIT == MG_INIT_INTERP0) {
-        const MGLev& C = A.Lc;
-        for (int e = threadIdx.x; e < EC * EC; e += NT) {
-            const int ic = ci0 + e % EC, jc = cj0 + e / EC;
-            const bool v = ic >= 0 && ic < C.w && jc >= 0 && jc < C.h;
-#pragma unroll
-            for (int c = 0; c < 2; ++c) cp_async_el<R>(&sc[c][e], v ? &A.crse_in(ic, jc, c) : A.crse_in.p[c], v);
-        }
+    for (int t = threadIdx.x; t < 4 * E; t += 256) {
+        const int r = t >> 2;
+        sm[(t & 1) * C::PLANE + (r + 1) * RS + KP + ((t >> 1) & 1)] = R(0);
     }
-    cp_async_wait_all();
-    __syncthreads();
-    // inverse diagonals; the interpolated coarse correction added to the initial guess
+    R* phi = sm + (r0 + 1) * RS;
+    auto store = [&](int q, int e) {
+        if (r0 + q < E) {
+            phi[q * RS + (((q + e) & 1) ? own1 : own0)] = u[0][q][e];
+            phi[C::PLANE + q * RS + (((q + e) & 1) ? own1 : own0)] = u[1][q][e];
+        }
+    };
+    if (INIT != MG_INIT_ZERO) {
+        if (act) {
 #pragma unroll
-    for (int e0 = 0; e0 < E * E; e0 += NT) {
-        const int e = e0 + threadIdx.x;
-        if (e >= E * E) break;
-        const int i = ti0 + e % E, j = tj0 + e / E;
-        const bool v = i >= L.vlo && i <= L.vhi_i && j >= L.vlo && j <= L.vhi_j;
-        sinv[e] = v ? mg_diag_inv<R, CELL>(L, i, j, sa[e], A.facx, A.facy) : R(0);
-        if ((INIT == MG_INIT_INTERP || INIT == MG_INIT_INTERP0) && v) {
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                const R* q = sc[c];
-                sp[c][e] = sp[c][e] + mg_interp1f<R, CELL>([&](int ic, int jc) { return q[(jc - cj0) * EC + (ic - ci0)]; }, i, j);
-            }
+            for (int q = 0; q < RT; ++q) store(q, 1);
         }
     }
     __syncthreads();
-    // colour sweeps over the interior of the loaded region (its outer ring stays fixed): only
-    // the points of the sweep's colour are visited, (E-2)/2 per row
-    constexpr int HW = (E - 2) / 2;
-    for (int s = 0; s < NSW; ++s) {
+    // value a sweep of colour e gives the point (cell-centred: 4/3 of the inner neighbours in the first
+    // and last column and row)
+    auto relaxed = [&](int q, int e, int c) -> R {
+        const int own = ((q + e) & 1) ? own1 : own0, out = ((q + e) & 1) ? out1 : out0;
+        const R* p = phi + c * C::PLANE;
+        R h = u[c][q][1 - e] + p[q * RS + out];
+        R a, b;
+        if (q > 0) a = u[c][q > 0 ? q - 1 : 0][1 - e]; else a = p[-RS + own];
+        if (q < RT - 1) b = u[c][q < RT - 1 ? q + 1 : q][1 - e]; else b = p[RT * RS + own];
+        R v = a + b;
+        if (CELL) {
+            const int i = ti0 + column(q, e), j = tj0 + r0 + q;
+            if (i == 0 || i == L.w - 1) h *= R(4. / 3.);
+            if (j == 0 || j == L.h - 1) v *= R(4. / 3.);
+        }
+        const R w = fma(ratio, v, h);
+        return fma(cx[q][e], w, LOW ? fma(low[q][e], w, rv[c][q][e]) : rv[c][q][e]);
+    };
+    auto sweep = [&](auto colour, bool zero) {
+        constexpr int e = decltype(colour)::value;
+        if (act) {
+            if (e == 0 && zero) {
 #pragma unroll
-        for (int q0 = 0; q0 < (E - 2) * HW; q0 += NT) {
-            const int q = q0 + threadIdx.x;
-            if (q >= (E - 2) * HW) break;
-            const int lj = 1 + q / HW, k = q - (lj - 1) * HW;
-            const int par = (s + ti0 + tj0 + lj) & 1;  // parity of li for (i + j + s) even
-            const int li = (par ? 1 : 2) + 2 * k;
-            const int i = ti0 + li, j = tj0 + lj;
-            if (i < L.vlo || i > L.vhi_i || j < L.vlo || j > L.vhi_j) continue;
-            const int e = lj * E + li;
-            const R inv = sinv[e];
+                for (int q = 0; q < RT; ++q) { u[0][q][0] = rv[0][q][0]; u[1][q][0] = rv[1][q][0]; }
+            } else {
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                const R* qq = sp[c];
-                sp[c][e] = mg_gs_inv<R, CELL>(L, i, j, qq[e - 1], qq[e + 1], qq[e - E], qq[e + E], srh[c][e], inv, A.facx, A.facy);
+                for (int q = 0; q < RT; ++q) { u[0][q][e] = relaxed(q, e, 0); u[1][q][e] = relaxed(q, e, 1); }
             }
+#pragma unroll
+            for (int q = 0; q < RT; ++q) store(q, e);
         }
         __syncthreads();
+    };
+#pragma unroll 1
+    for (int s = 0; s < NSW; s += 2) {
+        sweep(std::integral_constant<int, 0>{}, s == 0 && INIT == MG_INIT_ZERO);
+        sweep(std::integral_constant<int, 1>{}, false);
     }
-    if (RES) {
-        for (int e = threadIdx.x; e < Q * Q; e += NT) {
-            const int ri = e % Q, rj = e / Q;
-            const int i = t0i - 1 + ri, j = t0j - 1 + rj;
-            const bool v = i >= L.vlo && i <= L.vhi_i && j >= L.vlo && j <= L.vhi_j;
-            const bool in_tile = ri >= 1 && ri <= T && rj >= 1 && rj <= T;
-            const int k = (rj + H - 1) * E + (ri + H - 1);
+    if (act) {
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                R r = R(0);
-                if (v) {
-                    const R* q = sp[c];
-                    const R rh = srh[c][k];
-                    r = rh + sa[k] * q[k] - mg_lap<R, CELL>(L, i, j, q[k], q[k - 1], q[k + 1], q[k - E], q[k + E], A.facx, A.facy);
-                    if (NORM != MG_NORM_NONE && in_tile) {
-                        bmax = fmax(bmax, fabs((double)r));
-                        if (NORM == MG_NORM_FIRST) brhs = fmax(brhs, fabs((double)rh));
+        for (int q = 0; q < RT; ++q) {
+            const int lj = r0 + q;
+            const bool row = lj >= H && lj < H + T && tj0 + lj <= L.vhi_j;
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int li = column(q, e);
+                const bool in = row && li >= H && li < H + T && ti0 + li <= L.vhi_i;
+                if (RES && e == 0) {
+                    // (colour 0 in shared memory is not read by any other thread's residual)
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) {
+                        const R r = c0[q] * (relaxed(q, 0, c) - u[c][q][0]);
+                        if (lj < E) phi[c * C::PLANE + q * RS + ((q & 1) ? own1 : own0)] = r;
+                        if (NORM != MG_NORM_NONE && in) bmax = fmax(bmax, fabs((double)r));
                     }
                 }
-                sr[c][e] = r;
+                if (in) {
+                    vout(ti0 + li, tj0 + lj, 0) = u[0][q][e];
+                    vout(ti0 + li, tj0 + lj, 1) = u[1][q][e];
+                }
             }
         }
-    }
-    for (int e = threadIdx.x; e < T * T; e += NT) {
-        const int li = e % T, lj = e / T;
-        const int i = t0i + li, j = t0j + lj;
-        if (i > L.vhi_i || j > L.vhi_j) continue;
-        const int k = (lj + H) * E + (li + H);
-        vout(i, j, 0) = sp[0][k];
-        vout(i, j, 1) = sp[1][k];
     }
     if (RESTR) {
         __syncthreads();
-        const MGLev& C = A.Lc;
+        const MGLev& Lc = A.Lc;
         // coarse points whose centre 2I lies in this tile
-        const int ci0 = max(C.vlo, (t0i + 1) >> 1), cj0 = max(C.vlo, (t0j + 1) >> 1);
-        const int ci1 = min(C.vhi_i, (t0i + T - 1) >> 1), cj1 = min(C.vhi_j, (t0j + T - 1) >> 1);
-        const int cw = ci1 - ci0 + 1, ch = cj1 - cj0 + 1;
-        if (cw > 0 && ch > 0) {
-            for (int e = threadIdx.x; e < cw * ch; e += NT) {
-                const int I = ci0 + e % cw, J = cj0 + e / cw;
+        const int ci0 = max(Lc.vlo, (t0i + 1) >> 1), cj0 = max(Lc.vlo, (t0j + 1) >> 1);
+        const int ci1 = min(Lc.vhi_i, (t0i + T - 1) >> 1), cj1 = min(Lc.vhi_j, (t0j + T - 1) >> 1);
+        for (int t = threadIdx.x; t < T * T / 4; t += 256) {
+            const int I = ci0 + t % (T / 2), J = cj0 + t / (T / 2);
+            if (I > ci1 || J > cj1) continue;
+            const int x = 2 * I - ti0, y = 2 * J - tj0;  // centre (node) or first cell in the region
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    // residual at fine (i, j) is sr[c][(j - t0j + 1) * Q + (i - t0i + 1)]
-                    auto f = [&](int i, int j) -> R { return sr[c][(j - t0j + 1) * Q + (i - t0i + 1)]; };
-                    R v;
-                    if (CELL) {
-                        v = R(0.25) * (f(2 * I, 2 * J) + f(2 * I + 1, 2 * J) + f(2 * I, 2 * J + 1) + f(2 * I + 1, 2 * J + 1));
-                    } else {
-                        v = R(1. / 16.) * (f(2 * I - 1, 2 * J - 1) + R(2.) * f(2 * I, 2 * J - 1) + f(2 * I + 1, 2 * J - 1) +
-                                           R(2.) * f(2 * I - 1, 2 * J) + R(4.) * f(2 * I, 2 * J) + R(2.) * f(2 * I + 1, 2 * J) +
-                                           f(2 * I - 1, 2 * J + 1) + R(2.) * f(2 * I, 2 * J + 1) + f(2 * I + 1, 2 * J + 1));
-                    }
-                    A.crse_res(I, J, c) = v;
-                }
+            for (int c = 0; c < 2; ++c) {
+                auto f = [&](int li, int lj) -> R {
+                    return sm[c * C::PLANE + (lj + 1) * RS + ((li & 1) ? KP + 2 : 0) + (li >> 1)];
+                };
+                A.crse_res(I, J, c) = CELL ? R(0.25) * (f(x, y) + f(x + 1, y + 1))
+                                           : R(1. / 16.) * ((f(x - 1, y - 1) + f(x + 1, y - 1)) +
+                                                            (f(x - 1, y + 1) + f(x + 1, y + 1)) + R(4.) * f(x, y));
             }
         }
     }
