@@ -50,8 +50,8 @@ def test_cluster_form_equals_tile_form(nx, ny, precision, tol):
     try:
         b, cb = run(text, precision, "tiles")
     except hp.HpqError:
-        # FP32 V-cycles of very flat cells: the tile form's residual, formed at both colours, stalls at its
-        # rounding above the tolerance; the cluster form converges
+        # FP32 V-cycles of very flat cells: the tile form may stall at its rounding above the tolerance; the
+        # cluster form converges
         assert (nx, ny, precision, tol) == (511, 63, hp.MIXED, 1e-4)
         return
     # a V-cycle more or less where a norm meets the target to rounding
