@@ -24,6 +24,7 @@
 
 #include "common.cuh"
 #include "kernels.cuh"
+#include "mgcl_plan.hpp"
 
 namespace hpq {
 
@@ -34,11 +35,6 @@ struct MV {
     int pitch;
     int off;
     __device__ R& operator()(int i, int j, int c) const { return p[c][(ptrdiff_t)(j + off) * pitch + (i + off)]; }
-};
-
-struct MGLev {
-    int w, h;               // full box (cell: n; node: N+2)
-    int vlo, vhi_i, vhi_j;  // valid box [vlo, vhi]
 };
 
 template <class R, bool CELL>
@@ -1516,19 +1512,7 @@ public:
     void init(int nx, int ny, double dx_, double dy_) {
         dx = dx_; dy = dy_;
         cell = (nx % 2 == 0);
-        int lx, ly;
-        if (cell) { lx = nx - 1; ly = ny - 1; } else { lx = nx + 1; ly = ny + 1; }
-        for (int l = 0; l < 40; ++l) {
-            MGLev L;
-            L.w = lx + 1; L.h = ly + 1;
-            if (cell) { L.vlo = 0; L.vhi_i = lx; L.vhi_j = ly; }
-            else { L.vlo = 1; L.vhi_i = lx - 1; L.vhi_j = ly - 1; }
-            lev.push_back(L);
-            const int len_x = lx + 1, len_y = ly + 1, minw = cell ? 2 : 4;
-            if (len_x < 2 * minw || len_y < 2 * minw) break;
-            if (cell) { if (len_x % 2 || len_y % 2) break; lx = len_x / 2 - 1; ly = len_y / 2 - 1; }
-            else { if (lx % 2 || ly % 2) break; lx /= 2; ly /= 2; }
-        }
+        lev = mg_levels(nx, ny);
         nl = (int)lev.size();
         if (nl < 2) throw CudaError("hpmg: the domain cannot be coarsened (need at least 2 levels)");
         // single-block levels: from the first level (>= 1) whose hierarchy fits 160 KB of shared memory
@@ -1553,10 +1537,7 @@ public:
             bottom_smem1 = 0;
         }
         coarse.nl = nl - sb;
-        // the bottom solve of HpMultiGrid's CPU build (HpMultiGrid.cpp:1584-1592): 16 sweeps, or
-        // the longest side of the coarsest level rounded up to an even count when that is more
-        // (grids that stop coarsening early, e.g. 100 x 72 -> 25 x 18)
-        coarse.ns_bottom = std::max(16, (std::max(lev[nl - 1].w, lev[nl - 1].h) + 1) / 2 * 2);
+        coarse.ns_bottom = mg_bottom_sweeps(lev);
         // HPQ_MG_WARP=1 in the environment runs the smallest coarse levels on one warp (measured
         // slower at 255^2: 10.8 us instead of 7.0 for levels 9^2 and 5^2, so off by default)
         const char* ew = getenv("HPQ_MG_WARP");
@@ -1605,13 +1586,7 @@ public:
         cudaFuncAttributes fa{};
         HPQ_CUDA(cudaFuncGetAttributes(&fa, kern));
         const size_t limit = 227 * 1024 - fa.sharedSizeBytes;
-        // a whole component in one block where it fits (63^2 in double): a sweep then ends with a
-        // block barrier (45 cycles) instead of a cluster barrier (500); else the largest cluster. A
-        // level runs in block 0 where its points there cost less than a cluster barrier, as far
-        // as the shared memory reaches.
-        struct Try { int cs, own; };
-        const Try tries[] = {{1, 1 << 30}, {16, 4225}, {16, 1100}, {16, 300}, {8, 4225}, {8, 1100}, {8, 300}};
-        for (const Try& t : tries) {
+        for (const ClTry& t : kClTries) {
             if (!ClPlan<RS>::layout(pl.a, pl.smem, lev, dx, dy, t.cs, t.own, coarse.ns_bottom) || pl.smem > limit) continue;
             HPQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
             HPQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
