@@ -122,7 +122,9 @@ struct ClPlan {
             L.facy = (R)(1. / ((dy * f) * (dy * f)));
         }
         // rows per block: even on the last split level, doubled on every finer one, so that a
-        // block's coarse rows lie under its fine rows, and a multiple of the rows per thread
+        // block's coarse rows lie under its fine rows, a multiple of the rows per thread, and enough for
+        // every level (a node-centred level has 2 n + 1 rows over n, one more than doubling gives where
+        // the last split level fills its blocks)
         auto rows_per_thread = [&](const ClLev<R>& L, int rows) {
             const int groups = kClThreads / L.kp;
             int rt = 1;
@@ -136,7 +138,7 @@ struct ClPlan {
             for (int l = 0; l < nd; ++l) {
                 const int rp = base << (nd - 1 - l), rt = rows_per_thread(A.lev[l], rp);
                 if (!rt) return false;
-                if (rp % rt) fits = false;
+                if (rp % rt || cs * rp < A.lev[l].ny) fits = false;
             }
             if (!fits) base += 2;
         }

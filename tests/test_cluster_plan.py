@@ -1,0 +1,84 @@
+"""The shared-memory plan of the cluster multigrid over all grids: every row of every level belongs to a
+block, and the rows that the kernel reads and writes lie inside their planes. Plain C++, no GPU."""
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+CHECK = r"""
+#include <cstdio>
+#include "mgcl_plan.hpp"
+using namespace hpq;
+
+static long plans = 0, bad = 0;
+static void fail(const char* what, int nx, int ny, int bytes, const ClTry& t, int l, long a, long b) {
+    if (bad++ < 10) std::printf("%d x %d, %d bytes, cluster %d, own %d: level %d %s: %ld, %ld\n", nx, ny, bytes, t.cs, t.own, l, what, a, b);
+}
+
+template <class R>
+void check(int nx, int ny) {
+    const std::vector<MGLev> lev = mg_levels(nx, ny);
+    for (const ClTry& t : kClTries) {
+        ClArgs<R> A;
+        size_t smem = 0;
+        // (227 KB: the most that a block can have)
+        if (!ClPlan<R>::layout(A, smem, lev, 1.0, 1.0, t.cs, t.own, mg_bottom_sweeps(lev)) || smem > 227 * 1024) continue;
+        ++plans;
+        const int cs = A.cs;
+        auto err = [&](const char* what, int l, long a, long b) { fail(what, nx, ny, (int)sizeof(R), t, l, a, b); };
+        for (int l = 0; l < A.nl; ++l) {
+            const ClLev<R>& L = A.lev[l];
+            const int blocks = L.dist ? cs : 1, rs = 2 * L.kp + 2;
+            if ((long)blocks * L.rp < L.ny) err("rows without a block", l, (long)blocks * L.rp, L.ny);
+            if (2 * L.kp < L.nx || L.rt * L.ng != L.rp || L.kp * L.ng > kClThreads) err("threads", l, L.kp, L.ng);
+            for (int x = 0; x < kClThreads; ++x)
+                if ((int)((x * L.magic) >> 22) != x / L.kp) err("division by kp", l, x, L.kp);
+            // (a neighbour below exists where rows are sent to it)
+            for (int rank = 0; rank < blocks; ++rank)
+                if (cs > 1 && L.dist && (rank + 1) * L.rp < L.ny && rank + 1 >= cs) err("neighbour", l, rank, L.rp);
+            if (l <= A.lm) {
+                if (L.phi + (size_t)(L.rp + 2) * rs > A.elems || L.rhs + (size_t)L.rp * 2 * L.kp > A.elems) err("plane", l, L.phi, A.elems);
+                if (L.phi < A.coef_elems) err("plane in the coefficients", l, L.phi, A.coef_elems);
+            }
+            if (l + 1 == A.nl || l >= A.lm) continue;
+            const ClLev<R>& C = A.lev[l + 1];
+            if (L.dist && C.dist && cs > 1 && L.rp != 2 * C.rp) err("rows not doubled", l, L.rp, C.rp);
+            for (int rank = 0; rank < blocks; ++rank)
+                for (int q = 0; q < L.rp; ++q) {
+                    const int row = (L.dist ? rank * L.rp : 0) + q;
+                    // coarse rows that restriction writes
+                    if (row % 2 == 0 && row / 2 < C.ny) {
+                        const int d = row / 2 - (L.dist && C.dist ? rank * (L.rp / 2) : 0);
+                        if (d < 0 || d >= C.rp) err("restriction to row", l, row, d);
+                    }
+                }
+        }
+    }
+}
+
+int main() {
+    for (int nx = 3; nx <= 1100; ++nx)
+        for (int ny = 4 - nx % 2; ny <= (nx <= 400 ? 1100 : 420); ny += 2) {
+            if (mg_levels(nx, ny).size() < 2) continue;
+            check<double>(nx, ny);
+            check<float>(nx, ny);
+        }
+    std::printf("%ld plans, %ld faults\n", plans, bad);
+    return bad != 0 || plans < 10000;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def check(tmp_path_factory):
+    d = tmp_path_factory.mktemp("plan")
+    src = d / "check.cpp"
+    src.write_text(CHECK)
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-I", os.path.join(ROOT, "hipace2_b200", "csrc"), "-o", str(d / "check"), str(src)])
+    return subprocess.run([str(d / "check")], capture_output=True, text=True)
+
+
+def test_every_row_has_a_block_and_every_access_a_plane(check):
+    assert check.returncode == 0, check.stdout
