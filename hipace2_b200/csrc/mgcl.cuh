@@ -290,12 +290,13 @@ struct ClSolve {
             // columns (between two coarse columns)
             const int a1 = (k & 1) ? C.kp + 2 + (k >> 1) : (k >> 1);              // coarse column k
             const int a0 = (k & 1) ? ((k - 1) >> 1) : C.kp + 2 + ((k - 1) >> 1);  // coarse column k - 1
-            const R* cb = sm + cphi + rsc - (DIST && cdist ? rank * (rp / 2) : 0) * rsc;
+            const R* cb = sm + cphi + rsc;
+            const int cbase = DIST && cdist ? rank * (rp / 2) : 0, crp = C.rp;
             if (t.act) {
 #pragma unroll
                 for (int q = 0; q < RT; ++q) {
                     const int row = t.grow + q;
-                    const R* c1 = cb + (row >> 1) * rsc;
+                    const R* c1 = cb + cl_coarse_row(row, cbase, crp) * rsc;
                     R a;
                     if (CELL) a = c1[a1];
                     else a = (row & 1) ? (c1[a0] + c1[a1]) * R(0.5) : (c1[a1 - rsc] + c1[a1]) * R(0.5);

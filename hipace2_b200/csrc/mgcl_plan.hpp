@@ -87,6 +87,17 @@ struct ClArgs {
     unsigned elems, celems;    // shared-memory elements in use (solve, k_mg_cluster_coef)
 };
 
+// Row of a block's coarse plane (rows -1 .. crp) that interpolation reads for fine row `row`; base: the
+// plane's first row. A thread may own rows beyond the grid, for which the plane of a level in block 0
+// has none: it reads the last row's (and discards the value).
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline int cl_coarse_row(int row, int base, int crp) {
+    const int c = (row >> 1) - base;
+    return c < crp ? c : crp;
+}
+
 // Clusters tried in this order: a whole component in one block where it fits (63^2 in double): a sweep
 // then ends with a block barrier (45 cycles) instead of a cluster barrier (500); else the largest
 // cluster. A level runs in block 0 where its points there cost less than a cluster barrier, as far as

@@ -74,3 +74,10 @@ def test_cluster_form_equals_tile_form(nx, ny, precision, tol):
 @pytest.mark.parametrize("precision", [hp.PLAIN_FP64, hp.MIXED])
 def test_grids_whose_levels_are_all_split(nx, ny, tol, precision):
     test_cluster_form_equals_tile_form(nx, ny, precision, tol)
+
+
+# flat grids: blocks own more rows than the grid has, over a coarse level that lies in block 0
+@pytest.mark.parametrize("nx,ny", [(587, 31), (571, 31)])
+@pytest.mark.parametrize("precision", [hp.PLAIN_FP64, hp.MIXED])
+def test_flat_grids_with_rows_beyond_the_grid(nx, ny, precision):
+    test_cluster_form_equals_tile_form(nx, ny, precision, 0.3)

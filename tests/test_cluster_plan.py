@@ -45,9 +45,13 @@ void check(int nx, int ny) {
             if (l + 1 == A.nl || l >= A.lm) continue;
             const ClLev<R>& C = A.lev[l + 1];
             if (L.dist && C.dist && cs > 1 && L.rp != 2 * C.rp) err("rows not doubled", l, L.rp, C.rp);
+            // interpolation: rows of the coarse plane that the threads of every block read, in rows of that
+            // block's plane, which holds rows -1 .. C.rp
             for (int rank = 0; rank < blocks; ++rank)
                 for (int q = 0; q < L.rp; ++q) {
                     const int row = (L.dist ? rank * L.rp : 0) + q;
+                    const int c = cl_coarse_row(row, L.dist && C.dist ? rank * (L.rp / 2) : 0, C.rp);
+                    if (c - 1 < -1 || c > C.rp) err("interpolation from row", l, row, c);
                     // coarse rows that restriction writes
                     if (row % 2 == 0 && row / 2 < C.ny) {
                         const int d = row / 2 - (L.dist && C.dist ? rank * (L.rp / 2) : 0);
