@@ -5,8 +5,9 @@
 // frameworks that own the device memory pool and forbid side allocations, and real-time loops
 // that must not pay for or fail on an allocation at solve time. This entry point serves them:
 // the caller passes the right-hand side and the solution buffer; the transformed intermediate of
-// the solve lives in one file-scope device array of fixed size (the FFT twiddles of every length in
-// another, filled when the device is set up; the eigenvalues are formed where they are used). CUDA loads the library's device code lazily, so the array's
+// the solve lives in one file-scope device array of fixed size (the FFT twiddles of every length are
+// constant data beside it; the eigenvalues are formed where they are used). CUDA loads the
+// library's device code lazily, so the array's
 // memory is committed on a device by the first call on that device (which can therefore fail
 // with HPQ_ERR_CUDA when the device is already full) and held until the process exits.
 //
@@ -21,7 +22,6 @@
 // is made.
 #include <cuda_runtime.h>
 
-#include <cmath>
 #include <mutex>
 
 #include "../../include/hpq.h"
@@ -31,11 +31,68 @@ namespace {
 
 constexpr int kMaxN = 1023;
 constexpr size_t kPlane = (size_t)kMaxN * kMaxN;          // one nx x ny plane
-constexpr size_t kTw = 2048;                               // complex twiddles of M = 64 .. 2048, M/2 each
-constexpr size_t kScratchDoubles = 2 * kPlane + 2 * kTw;   // work plane (the rest is not used)
+constexpr size_t kTw = 2016;                               // complex twiddles of M = 64 .. 2048, M/2 each
+constexpr size_t kScratchDoubles = 2 * kPlane + 2 * 2048;  // work plane (the rest is not used)
 
 static __device__ __align__(256) double g_poisson_scratch[kScratchDoubles];
-static __device__ __align__(256) double g_poisson_twiddles[2 * kTw];
+// Twiddles exp(-2 pi i k / M), k < M/2, of M = 64 .. 2048 in this order, as constant data of the
+// library's device code: they are there whichever stream or capture makes the first call. Formed by
+// the compiler: the Taylor series of sine and cosine on [0, pi/4] in pairs of doubles (Dekker, "A
+// floating-point technique for extending the available precision", 1971), then symmetry.
+struct Pair {
+    double hi, lo;
+};
+constexpr Pair two_sum(double a, double b) {
+    const double s = a + b, t = s - a;
+    return {s, (a - (s - t)) + (b - t)};
+}
+constexpr Pair two_mul(double a, double b) {
+    const double c = 134217729.0;  // 2^27 + 1
+    const double ah = c * a - (c * a - a), al = a - ah, bh = c * b - (c * b - b), bl = b - bh, p = a * b;
+    return {p, ((ah * bh - p) + ah * bl + al * bh) + al * bl};
+}
+constexpr Pair add(Pair a, Pair b) {
+    const Pair s = two_sum(a.hi, b.hi);
+    return two_sum(s.hi, s.lo + a.lo + b.lo);
+}
+constexpr Pair mul(Pair a, Pair b) {
+    const Pair p = two_mul(a.hi, b.hi);
+    return two_sum(p.hi, p.lo + (a.hi * b.lo + a.lo * b.hi));
+}
+constexpr Pair over(Pair a, double n) {  // a / n
+    const double q = a.hi / n;
+    const Pair p = two_mul(q, n);
+    return two_sum(q, (((a.hi - p.hi) - p.lo) + a.lo) / n);
+}
+struct Twiddles {
+    double v[2 * kTw];
+};
+constexpr size_t tw_offset(int M) { return (size_t)M / 2 - 32; }  // 32 + 64 + .. + M/4 before length M
+constexpr Twiddles make_twiddles() {
+    Twiddles t{};
+    double c[257] = {}, s[257] = {};  // cos, sin of 2 pi k / 2048 in the first octant
+    for (int k = 0; k <= 256; ++k) {
+        const Pair x = mul({3.14159265358979323846, 1.2246467991473532e-16}, {k / 1024.0, 0.0}), x2 = mul(x, x);
+        Pair p{1.0, 0.0}, q = x, sc{0.0, 0.0}, ss{0.0, 0.0};
+        for (int n = 0; n < 12; ++n) {  // terms 2n and 2n + 1; the first one left out is below 1e-26
+            sc = add(sc, p);
+            ss = add(ss, q);
+            p = over(mul(p, x2), -(2.0 * n + 1) * (2 * n + 2));
+            q = over(mul(q, x2), -(2.0 * n + 2) * (2 * n + 3));
+        }
+        c[k] = sc.hi;
+        s[k] = ss.hi;
+    }
+    for (int M = 64; M <= 2048; M *= 2)
+        for (int k = 0; k < M / 2; ++k) {
+            const int a = k * (2048 / M), h = a <= 512 ? a : 1024 - a;  // angle, folded into the first quarter
+            const double co = h <= 256 ? c[h] : s[512 - h], si = h <= 256 ? s[h] : c[512 - h];
+            t.v[2 * (tw_offset(M) + k)] = a <= 512 ? co : -co;
+            t.v[2 * (tw_offset(M) + k) + 1] = -si;
+        }
+    return t;
+}
+static __device__ __align__(256) const Twiddles g_poisson_twiddles = make_twiddles();
 
 constexpr int kMaxDevices = 64;
 std::mutex g_mutex;
@@ -44,21 +101,10 @@ const hpq::Cx<double>* g_twiddle_ptr[kMaxDevices] = {};
 
 cudaError_t set_smem_attributes();
 
-// Set-up, once per device with that device current: the host address of the array is only a
-// stand-in, kernels must be given the device address returned here. The shared-memory limits of
-// the pass kernels are raised and the twiddles written at the same time, so later calls make no
-// set-up call at all.
-size_t tw_offset(int M) { return (size_t)M / 2 - 32; }  // 32 + 64 + .. + M/4 before length M
-cudaError_t fill_twiddles(void* dst) {
-    static double h[2 * kTw];  // (under the mutex)
-    const double pi = 3.14159265358979323846;
-    for (int M = 64; M <= 2048; M *= 2)
-        for (int k = 0; k < M / 2; ++k) {
-            h[2 * (tw_offset(M) + k)] = std::cos(2 * pi * k / M);
-            h[2 * (tw_offset(M) + k) + 1] = -std::sin(2 * pi * k / M);
-        }
-    return cudaMemcpy(dst, h, sizeof(h), cudaMemcpyHostToDevice);
-}
+// Set-up, once per device with that device current: the host addresses of the arrays are only
+// stand-ins, kernels must be given the device addresses returned here. The shared-memory limits of
+// the pass kernels are raised at the same time, so later calls make no set-up call at all. Nothing
+// is copied or launched, so that no stream has to wait for it.
 int scratch_for_current_device(double** out, const hpq::Cx<double>** tw) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return HPQ_ERR_CUDA;
@@ -69,7 +115,6 @@ int scratch_for_current_device(double** out, const hpq::Cx<double>** tw) {
         if (set_smem_attributes() != cudaSuccess) return HPQ_ERR_CUDA;
         void* t = nullptr;
         if (cudaGetSymbolAddress(&t, g_poisson_twiddles) != cudaSuccess || !t) return HPQ_ERR_CUDA;
-        if (fill_twiddles(t) != cudaSuccess) return HPQ_ERR_CUDA;
         g_twiddle_ptr[dev] = static_cast<const hpq::Cx<double>*>(t);
         g_scratch_ptr[dev] = static_cast<double*>(p);
     }
