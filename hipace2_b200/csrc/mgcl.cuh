@@ -707,6 +707,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_mg_cluster_coef(const __grid_
             }
         }
     }
+    __syncthreads();  // (the last level's diagonals, where it is split, are behind no other barrier)
     R* out = P.coef + (size_t)rank * P.coef_elems;
     for (int l = 0; l < (rank == 0 ? min(P.nl, P.lm) : nd); ++l) {
         const ClLev<R>& L = slev[l];

@@ -67,10 +67,10 @@ def test_cluster_form_equals_tile_form(nx, ny, precision, tol):
         assert np.linalg.norm(a[k] - b[k]) <= bound * np.linalg.norm(b[k]), k
 
 
-# every level split over the cluster, the coarsest with an even number of rows: a finer level has one row more than
-# twice as many. Most of these coarsen once only and converge slowly (0.9 per V-cycle): a loose tolerance
-@pytest.mark.parametrize("nx,ny,tol", [(263, 263, 1e-4), (193, 193, 0.05), (257, 257, 0.05), (257, 193, 0.05), (321, 65, 0.05),
-                                       (65, 321, 0.05)])
+# every level split over the cluster: cell-centred, and node-centred with an even number of rows on the coarsest
+# level (a finer level has one row more than twice as many)
+@pytest.mark.parametrize("nx,ny,tol", [(194, 194, 1e-4), (226, 150, 1e-4), (263, 263, 1e-4), (193, 193, 0.05), (257, 257, 0.05),
+                                       (257, 193, 0.05), (321, 65, 0.05), (65, 321, 0.05)])
 @pytest.mark.parametrize("precision", [hp.PLAIN_FP64, hp.MIXED])
 def test_grids_whose_levels_are_all_split(nx, ny, tol, precision):
     test_cluster_form_equals_tile_form(nx, ny, precision, tol)
