@@ -219,8 +219,8 @@ struct ClSolve {
         const int rh0 = par ? kp + k : k, rh1 = par ? k : kp + k;
         R* phi = sm + L.phi + (t.r0 + 1) * rs;
         // neighbours of this block on the level, and this thread's share in the exchange with them
-        const bool has_up = DIST && cs > 1 && rank > 0 && rank * rp < lny;
-        const bool has_dn = DIST && rank + 1 < cs && (rank + 1) * rp < lny;
+        const bool has_up = DIST && cl_joined(rank, cs, rp, lny, CELL);
+        const bool has_dn = DIST && cl_joined(rank + 1, cs, rp, lny, CELL);
         const bool top = has_up && t.act && t.r0 == 0;
         const bool bot = has_dn && t.act && t.r0 + RT == rp;
         int nu = 0, nd = 0;

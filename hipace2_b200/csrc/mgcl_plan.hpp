@@ -87,6 +87,14 @@ struct ClArgs {
     unsigned elems, celems;    // shared-memory elements in use (solve, k_mg_cluster_coef)
 };
 
+// Whether block `rank` exchanges rows of a level split into `rp` rows per block with the block above it. A
+// node-centred level counts one row beyond its last: the finer level has 2 n + 1 rows over n, and a block
+// with the last of them alone interpolates it from the row above, which lies in the block above.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline bool cl_joined(int rank, int cs, int rp, int ny, bool cell) { return rank > 0 && rank < cs && rank * rp < ny + (cell ? 0 : 1); }
+
 // Row of a block's coarse plane (rows -1 .. crp) that interpolation reads for fine row `row`; base: the
 // plane's first row. A thread may own rows beyond the grid, for which the plane of a level in block 0
 // has none: it reads the last row's (and discards the value).

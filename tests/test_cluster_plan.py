@@ -35,9 +35,12 @@ void check(int nx, int ny) {
             if (2 * L.kp < L.nx || L.rt * L.ng != L.rp || L.kp * L.ng > kClThreads) err("threads", l, L.kp, L.ng);
             for (int x = 0; x < kClThreads; ++x)
                 if ((int)((x * L.magic) >> 22) != x / L.kp) err("division by kp", l, x, L.kp);
-            // (a neighbour below exists where rows are sent to it)
-            for (int rank = 0; rank < blocks; ++rank)
-                if (cs > 1 && L.dist && (rank + 1) * L.rp < L.ny && rank + 1 >= cs) err("neighbour", l, rank, L.rp);
+            // blocks exchange rows with a neighbour that exists, across every pair of rows of the grid
+            for (int rank = 0; rank <= blocks; ++rank) {
+                const bool joined = L.dist && cl_joined(rank, cs, L.rp, L.ny, nx % 2 == 0);
+                if (joined && (rank == 0 || rank >= cs)) err("neighbour", l, rank, L.rp);
+                if (L.dist && rank > 0 && rank * L.rp < L.ny && !joined) err("no exchange", l, rank, L.rp);
+            }
             if (l <= A.lm) {
                 if (L.phi + (size_t)(L.rp + 2) * rs > A.elems || L.rhs + (size_t)L.rp * 2 * L.kp > A.elems) err("plane", l, L.phi, A.elems);
                 if (L.phi < A.coef_elems) err("plane in the coefficients", l, L.phi, A.coef_elems);
@@ -52,6 +55,9 @@ void check(int nx, int ny) {
                     const int row = (L.dist ? rank * L.rp : 0) + q;
                     const int c = cl_coarse_row(row, L.dist && C.dist ? rank * (L.rp / 2) : 0, C.rp);
                     if (c - 1 < -1 || c > C.rp) err("interpolation from row", l, row, c);
+                    // (a row of the block above is there if the two exchange rows of that level)
+                    if (L.dist && C.dist && row < L.ny && nx % 2 && row % 2 == 0 && row > 0 && c == 0 && !cl_joined(rank, cs, C.rp, C.ny, false))
+                        err("interpolation without the block above", l, row, rank);
                     // coarse rows that restriction writes
                     if (row % 2 == 0 && row / 2 < C.ny) {
                         const int d = row / 2 - (L.dist && C.dist ? rank * (L.rp / 2) : 0);
