@@ -1577,7 +1577,7 @@ public:
     // solve (tolerances below kRefineTol)
     ClPlan<R> cl;
     ClPlan<double> cl64;
-    unsigned long long* cl_slot = nullptr;  // ClArgs::slot
+    ClNorm* cl_slot = nullptr;  // ClArgs::slot
     void* cl_coef = nullptr;                // ClArgs::coef
 
     template <class IO, class RS, bool CELL>
@@ -1624,7 +1624,7 @@ public:
         const size_t bytes = std::max(cl.ok ? cl.a.cs * (size_t)cl.a.coef_elems * sizeof(R) : 0,
                                       cl64.ok ? cl64.a.cs * (size_t)cl64.a.coef_elems * sizeof(double) : 0);
         if (bytes) {
-            HPQ_CUDA(cudaMalloc(&cl_slot, 6 * kClMaxBlocks * sizeof(unsigned long long)));
+            HPQ_CUDA(cudaMalloc(&cl_slot, 6 * kClMaxBlocks * sizeof(ClNorm)));
             HPQ_CUDA(cudaMalloc(&cl_coef, bytes));
             HPQ_CUDA(cudaMemset(cl_coef, 0, bytes));
         }

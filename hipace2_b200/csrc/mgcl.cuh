@@ -679,7 +679,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_mg_cluster_coef(const __grid_
     cl_levels_to_shared(P, slev, 0);
     int4* z = reinterpret_cast<int4*>(cl_smem);
     for (unsigned t = threadIdx.x; t < P.celems * sizeof(R) / 16; t += kClThreads) z[t] = make_int4(0, 0, 0, 0);
-    if (rank == 0 && threadIdx.x < 6 * kClMaxBlocks) P.slot[threadIdx.x] = 0;
+    if (rank == 0 && threadIdx.x < 6 * kClMaxBlocks) P.slot[threadIdx.x] = ClNorm{};
     __syncthreads();
     const S s{slev, nullptr, nullptr, P.nl, rank, cs, P.ns_bottom, P.lm, P.nm, P.matrix};
     int nd = 0;
@@ -780,9 +780,6 @@ __global__ void __launch_bounds__(kClThreads, 1)
     sync_all();  // every block has started: its shared memory may be written
     // largest |residual| of the block -> global; the decision is taken by block 0 of each cluster once
     // every block's value of the iteration is there
-    auto tagged = [](double v, int it) {
-        return ((unsigned long long)__double_as_longlong(v) & ~0xffffull) | (unsigned long long)(it + 1);
-    };
     auto block_max = [&](double v) {  // valid in thread 0
         const unsigned long long b = (unsigned long long)__double_as_longlong(v);
         const unsigned hi = (unsigned)(b >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
@@ -797,34 +794,41 @@ __global__ void __launch_bounds__(kClThreads, 1)
         return m;
     };
     const int me = comp * kClMaxBlocks + rank;
-    auto publish = [&](double worst, int it) {
+    auto publish = [&](double worst, ClNorm* slot, int it) {
         const double m = block_max(worst);
-        if (threadIdx.x == 0) *(volatile unsigned long long*)(P.slot + (it & 1) * 2 * kClMaxBlocks + me) = tagged(m, it);
+        if (threadIdx.x == 0) {
+            const ClNorm n = cl_norm((unsigned long long)__double_as_longlong(m), (unsigned)it + 1u);
+            volatile unsigned long long* w = slot[me].w;
+            w[0] = n.w[0];
+            w[1] = n.w[1];
+        }
     };
+    auto slots = [&](int it) { return P.slot + (it & 1) * 2 * kClMaxBlocks; };
+    ClNorm* const rhs_slots = P.slot + 4 * kClMaxBlocks;
     double target = 0, maxnorm = 0;  // warp 0 of block 0 of each cluster
     auto decide = [&](int it) {      // warp 0 of block 0 of each cluster
         const int lane = threadIdx.x & 31;
         int ok = 1;
         const int late = *(const volatile int*)&P.ctl->mgp_bar_err;  // (a wait of any block ran out)
-        auto fetch = [&](const unsigned long long* p, int tag) -> double {
-            unsigned long long v = 0;
+        auto fetch = [&](const ClNorm* p, int iteration) -> double {
+            ClNorm v{};
             if ((lane & 15) < cs) {
+                const volatile unsigned long long* w = p[lane].w;
                 for (long long n = 0;; ++n) {
-                    v = *(const volatile unsigned long long*)(p + lane);
-                    if ((v & 0xffffull) == (unsigned long long)tag) break;
+                    v = {{w[0], w[1]}};
+                    if (cl_norm_arrived(v, (unsigned)iteration + 1u)) break;
                     if ((n & 1023) == 1023 && *(const volatile int*)&P.ctl->mgp_bar_err) { ok = 0; break; }
                     if (n > kBarrierSpins) { atomicExch(&P.ctl->mgp_bar_err, 1); ok = 0; break; }
                 }
             }
             __syncwarp();
-            v &= ~0xffffull;
-            const unsigned hi = (unsigned)(v >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
-            const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)v : 0u);
+            const unsigned hi = cl_norm_hi(v), mh = __reduce_max_sync(0xffffffffu, hi);
+            const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? cl_norm_lo(v) : 0u);
             return __longlong_as_double((long long)(((unsigned long long)mh << 32) | ml));
         };
-        const double w = fetch(P.slot + (it & 1) * 2 * kClMaxBlocks, it + 1);
+        const double w = fetch(slots(it), it);
         if (it == 0) {
-            const double m = fetch(P.slot + 4 * kClMaxBlocks, 1);
+            const double m = fetch(rhs_slots, 0);
             maxnorm = m >= w ? m : w;
             target = fmax(P.tol_abs, fmax(P.tol_rel, 1.e-16) * maxnorm);
         }
@@ -850,11 +854,8 @@ __global__ void __launch_bounds__(kClThreads, 1)
     // consecutive sweeps. The norm of a V-cycle travels between the clusters while the next one
     // descends; a descent after the last V-cycle is thrown away.
     ClSeq seq{{0, 0}};
-    {
-        const double m = block_max(rmax);
-        if (threadIdx.x == 0) *(volatile unsigned long long*)(P.slot + 4 * kClMaxBlocks + me) = tagged(m, 0);
-    }
-    publish(s.template run_phase<true>(0, S::LOAD, 4, true, &seq), 0);
+    publish(rmax, rhs_slots, 0);
+    publish(s.template run_phase<true>(0, S::LOAD, 4, true, &seq), slots(0), 0);
     for (int it = 0;;) {
         if (nd == 1) {
             if (rank == 0 && threadIdx.x < 32) decide(it);
@@ -877,7 +878,8 @@ __global__ void __launch_bounds__(kClThreads, 1)
         }
         for (int l = (nd == P.nl ? nd - 2 : nd - 1); l >= 1; --l) s.template run_phase<true>(l, S::INTERP, 4, false, &seq);
         const double worst = s.template run_phase<true>(0, S::INTERP, 8, true, &seq);
-        publish(worst, ++it);
+        ++it;
+        publish(worst, slots(it), it);
     }
     if (sh.go == 0) {
         __syncthreads();

@@ -48,6 +48,26 @@ constexpr int kClMaxLevels = 12;
 constexpr int kClMaxBlocks = 16;  // per cluster
 constexpr int kClWarpScratch = 384;  // elements of matrix_column (levels of at most 32 storage places)
 
+// Host and device code of this file
+#ifdef __CUDACC__
+#define HPQ_HD __host__ __device__
+#else
+#define HPQ_HD
+#endif
+
+// A norm that a block publishes for the others: the upper and the lower 32 bits of the double, each in a
+// 64-bit word with the iteration number + 1, so that value and arrival are in the same store and the
+// two stores need no order
+struct ClNorm {
+    unsigned long long w[2];
+};
+HPQ_HD inline ClNorm cl_norm(unsigned long long bits, unsigned tag) {
+    return {{(bits & ~0xffffffffull) | tag, (bits << 32) | tag}};
+}
+HPQ_HD inline bool cl_norm_arrived(const ClNorm& n, unsigned tag) { return (unsigned)n.w[0] == tag && (unsigned)n.w[1] == tag; }
+HPQ_HD inline unsigned cl_norm_hi(const ClNorm& n) { return (unsigned)(n.w[0] >> 32); }
+HPQ_HD inline unsigned cl_norm_lo(const ClNorm& n) { return (unsigned)(n.w[1] >> 32); }
+
 // One level of the cluster form. Shared-memory planes (element offsets): a row of phi and xrow has
 // 2 kp + 2 elements: even columns at [k], a zero, a zero, odd columns at [kp + 2 + k] (the zeros are
 // the values outside the grid); phi has rp + 2 rows (halo rows above and below). rhs and inverse
@@ -76,9 +96,7 @@ struct ClArgs {
     ClLev<R> lev[kClMaxLevels];
     Ctl* ctl;
     double tol_rel, tol_abs;
-    // residual norm of every block by iteration parity, then |rhs|: the double's bits with the low 16
-    // replaced by iteration + 1, so that value and arrival are one 64-bit store (cleared per solve)
-    unsigned long long* slot;  // [3][2 * kClMaxBlocks]
+    ClNorm* slot;  // [3][2 * kClMaxBlocks]: norm of every block by iteration parity, then |rhs| (cleared per solve)
     // coefficient region of every block, in the order of its shared memory (from element 0): inverse
     // diagonals and coefficients of the split levels (dist_elems), in block 0 also those of its
     // own levels, then the matrix (coef_elems)
@@ -90,18 +108,12 @@ struct ClArgs {
 // Whether block `rank` exchanges rows of a level split into `rp` rows per block with the block above it. A
 // node-centred level counts one row beyond its last: the finer level has 2 n + 1 rows over n, and a block
 // with the last of them alone interpolates it from the row above, which lies in the block above.
-#ifdef __CUDACC__
-__host__ __device__
-#endif
-inline bool cl_joined(int rank, int cs, int rp, int ny, bool cell) { return rank > 0 && rank < cs && rank * rp < ny + (cell ? 0 : 1); }
+HPQ_HD inline bool cl_joined(int rank, int cs, int rp, int ny, bool cell) { return rank > 0 && rank < cs && rank * rp < ny + (cell ? 0 : 1); }
 
 // Row of a block's coarse plane (rows -1 .. crp) that interpolation reads for fine row `row`; base: the
 // plane's first row. A thread may own rows beyond the grid, for which the plane of a level in block 0
 // has none: it reads the last row's (and discards the value).
-#ifdef __CUDACC__
-__host__ __device__
-#endif
-inline int cl_coarse_row(int row, int base, int crp) {
+HPQ_HD inline int cl_coarse_row(int row, int base, int crp) {
     const int c = (row >> 1) - base;
     return c < crp ? c : crp;
 }

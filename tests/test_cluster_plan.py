@@ -9,6 +9,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 CHECK = r"""
 #include <cstdio>
+#include <cstring>
 #include "mgcl_plan.hpp"
 using namespace hpq;
 
@@ -75,6 +76,19 @@ int main() {
             check<double>(nx, ny);
             check<float>(nx, ny);
         }
+    // a norm keeps every bit on its way between the blocks, and is taken for another iteration's nowhere
+    for (double v : {0.0, 1.0, 1.0 / 3.0, 0x1.fffffffffffffp-30, 3.141592653589793e100, 5e-324}) {
+        unsigned long long b, r;
+        std::memcpy(&b, &v, 8);
+        for (unsigned tag : {1u, 2u, 201u, 65536u, 100001u}) {
+            const ClNorm n = cl_norm(b, tag);
+            r = ((unsigned long long)cl_norm_hi(n) << 32) | cl_norm_lo(n);
+            if (r != b || !cl_norm_arrived(n, tag) || cl_norm_arrived(n, tag + 1) || cl_norm_arrived(ClNorm{}, tag)) ++bad, std::printf("norm %a\n", v);
+            ClNorm half = n;  // (one of the two words still the older iteration's)
+            half.w[1] = cl_norm(b, tag + 2).w[1];
+            if (cl_norm_arrived(half, tag) || cl_norm_arrived(half, tag + 2)) ++bad, std::printf("half a norm\n");
+        }
+    }
     std::printf("%ld plans, %ld faults\n", plans, bad);
     return bad != 0 || plans < 10000;
 }
