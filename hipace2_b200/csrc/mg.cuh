@@ -1669,8 +1669,13 @@ public:
         ClArgs<RS> A = cluster_args(pl, ctl);
         A.tol_rel = tol_rel; A.tol_abs = tol_abs; A.maxiter = maxiter;
         cudaLaunchConfig_t cfg{};
-        cudaLaunchAttribute at[1];
+        cudaLaunchAttribute at[2];
         cluster_config(cfg, at, A.cs, pl.smem, st);
+        // both clusters resident or neither: each waits for the other's norms, and the clusters of other
+        // handles may hold the room of one of them
+        at[1].id = cudaLaunchAttributeCooperative;
+        at[1].val.cooperative = 1;
+        cfg.numAttrs = 2;
         HPQ_CUDA(cudaLaunchKernelEx(&cfg, k_mg_cluster<R, RS, CELL>, A, cluster_view(S, C_BX, C_BY), cluster_view(S, C_SY, C_SX)));
         HPQ_LAUNCH_CHECK();
     }
