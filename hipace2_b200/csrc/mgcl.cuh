@@ -798,9 +798,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
         const double m = block_max(worst);
         if (threadIdx.x == 0) {
             const ClNorm n = cl_norm((unsigned long long)__double_as_longlong(m), (unsigned)it + 1u);
-            volatile unsigned long long* w = slot[me].w;
-            w[0] = n.w[0];
-            w[1] = n.w[1];
+            asm volatile("st.volatile.global.v2.u64 [%0], {%1, %2};" ::"l"(slot + me), "l"(n.w[0]), "l"(n.w[1]) : "memory");
         }
     };
     auto slots = [&](int it) { return P.slot + (it & 1) * 2 * kClMaxBlocks; };
@@ -813,9 +811,8 @@ __global__ void __launch_bounds__(kClThreads, 1)
         auto fetch = [&](const ClNorm* p, int iteration) -> double {
             ClNorm v{};
             if ((lane & 15) < cs) {
-                const volatile unsigned long long* w = p[lane].w;
                 for (long long n = 0;; ++n) {
-                    v = {{w[0], w[1]}};
+                    asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];" : "=l"(v.w[0]), "=l"(v.w[1]) : "l"(p + lane) : "memory");
                     if (cl_norm_arrived(v, (unsigned)iteration + 1u)) break;
                     if ((n & 1023) == 1023 && *(const volatile int*)&P.ctl->mgp_bar_err) { ok = 0; break; }
                     if (n > kBarrierSpins) { atomicExch(&P.ctl->mgp_bar_err, 1); ok = 0; break; }

@@ -56,9 +56,9 @@ constexpr int kClWarpScratch = 384;  // elements of matrix_column (levels of at 
 #endif
 
 // A norm that a block publishes for the others: the upper and the lower 32 bits of the double, each in a
-// 64-bit word with the iteration number + 1, so that value and arrival are in the same store and the
-// two stores need no order
-struct ClNorm {
+// 64-bit word with the iteration number + 1, so that value and arrival are in the same word and the two
+// words may be seen in any order
+struct alignas(16) ClNorm {
     unsigned long long w[2];
 };
 HPQ_HD inline ClNorm cl_norm(unsigned long long bits, unsigned tag) {
