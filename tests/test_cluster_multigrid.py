@@ -47,13 +47,7 @@ def run(text, precision, form):
 def test_cluster_form_equals_tile_form(nx, ny, precision, tol):
     text = deck(nx, ny, tol)
     a, ca = run(text, precision, "cluster")
-    try:
-        b, cb = run(text, precision, "tiles")
-    except hp.HpqError:
-        # FP32 V-cycles of very flat cells: the tile form may stall at its rounding above the tolerance; the
-        # cluster form converges
-        assert (nx, ny, precision, tol) == (511, 63, hp.MIXED, 1e-4)
-        return
+    b, cb = run(text, precision, "tiles")
     # a V-cycle more or less where a norm meets the target to rounding
     assert cb > 0 and abs(ca - cb) <= max(1, cb // 20), (ca, cb)
     # rounding of a residual, eps 4/dx^2 |B|, against the smallest eigenvalue of the 12 x 12 box, 2 pi^2/144,
