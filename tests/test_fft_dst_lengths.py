@@ -1,5 +1,7 @@
 """The register FFT of the DST-I (radix-8 passes, then one of radix 8, 4 or 2) at every length it is
-compiled for, through the allocation-free Poisson solve against dense sine matrices."""
+compiled for, against dense sine matrices: M = 64 .. 2048 through the allocation-free Poisson solve
+(double), M = 64 .. 4096 and the Bluestein lengths L = 64 .. 8192 in both precisions through the
+slice loop's Psi solve."""
 import ctypes
 
 import numpy as np
@@ -42,3 +44,38 @@ def test_poisson_at_every_length(nx, ny):
         want = dense(f, dx, dy)
         # four transforms of log2(2(n+1)) <= 11 levels, a few roundings of 1.1e-16 each
         assert np.linalg.norm(u.cpu().numpy() - want) <= 4 * 11 * 4 * 1.1e-16 * np.linalg.norm(want)
+
+
+def smallest_eigenvalue(nx, ny, dx, dy):
+    return 4 * (np.sin(np.pi / (2 * (nx + 1))) ** 2 / dx ** 2 + np.sin(np.pi / (2 * (ny + 1))) ** 2 / dy ** 2)
+
+
+# radix-2 axes: M = 2(n + 1); Bluestein axes: L >= 4(n + 1) - 1, 64 128 256 512 1024 2048 4096 8192; each length on
+# the x axis (first and last pass) and on the y axis (eigenvalue pass)
+@pytest.mark.parametrize("nx,ny", [(31, 63), (127, 31), (63, 255), (255, 127), (511, 1023), (1023, 511), (2047, 31), (31, 2047),
+                                   (14, 20), (20, 14), (40, 100), (100, 40), (250, 320), (320, 250), (600, 1200), (1200, 600),
+                                   (2046, 34), (321, 63), (255, 41)])
+@pytest.mark.parametrize("precision", [hp.PLAIN_FP64, hp.MIXED])
+def test_psi_at_every_length_and_precision(nx, ny, precision, monkeypatch):
+    from cases import PC_SMALL
+    monkeypatch.setenv("HPQ_DST", "fft")  # (in single precision the default on some of these grids are the sine GEMMs)
+    text = (PC_SMALL.replace("amr.n_cell = 32 32 40", "amr.n_cell = %d %d 8" % (nx, ny))
+            .replace("beam.position_mean = 0. 0. 0.", "beam.position_mean = 0.7 -0.4 0."))
+    sim = hp.Hipace(text, precision=precision, graphs=False)
+    sim.init_data()
+    sim.begin_step(0)
+    for s in range(7, 3, -1):
+        sim.solve_one_slice(s)
+    f, psi = -sim.get_field("rhomjz"), sim.get_field("Psi")
+    for s in range(3, -1, -1):
+        sim.solve_one_slice(s)
+    sim.end_step()
+    sim.close()
+    dx, dy = 16.0 / nx, 16.0 / ny
+    want = dense(f, dx, dy)
+    assert np.linalg.norm(want) > 0
+    # four transforms, each of at most two FFTs of 13 levels and three products, two roundings a step; what they add
+    # to the lowest mode is divided by the smallest eigenvalue
+    eps = 1.1e-16 if precision == hp.PLAIN_FP64 else 6e-8
+    bound = 4 * 29 * 2 * eps * max(np.linalg.norm(want), np.linalg.norm(f) / smallest_eigenvalue(nx, ny, dx, dy))
+    assert np.linalg.norm(psi - want) <= bound, (np.linalg.norm(psi - want) / np.linalg.norm(want), bound / np.linalg.norm(want))

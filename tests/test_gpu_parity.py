@@ -459,8 +459,8 @@ def test_bluestein_dst_on_odd_grids_matches_oracle(monkeypatch):
     These grids also stop coarsening early (100 x 72 -> 25 x 18), so the multigrid's bottom level
     takes more than 16 sweeps (HpMultiGrid's CPU rule, which the oracle restates); with 16 the
     V-cycles differ and Bz, the curl of a nearly curl-free current in this weak wake, ends 4e-10
-    from the oracle. The library's default on these grids is the sine-GEMM form (faster below
-    1024 cells); HPQ_DST=fft selects the Bluestein FFT."""
+    from the oracle. The Bluestein FFT is the library's default on these grids in double precision;
+    HPQ_DST=fft selects it whatever the default is."""
     monkeypatch.setenv("HPQ_DST", "fft")
     for shape in ("100 72 24", "45 33 24"):
         text = (EXPLICIT_MOVING.replace("amr.n_cell = 33 33 40", "amr.n_cell = " + shape)
