@@ -12,7 +12,7 @@
 // with HPQ_ERR_CUDA when the device is already full) and held until the process exits.
 //
 // Limit: nx and ny of the form 2^k - 1 with 31 <= n <= 1023 (the shared-memory FFT path of the
-// DST-I), i.e. at most 1023 x 1023 cells; the scratch array is 16.1 MiB.
+// DST-I), i.e. at most 1023 x 1023 cells; the scratch array is 8.0 MiB.
 // All calls share the array and it keeps the contents of the last call. Every element a solve
 // reads is written earlier in the same solve, so nothing needs clearing between calls; two
 // calls whose kernels overlap on the GPU (different streams, or different host threads on one
@@ -32,9 +32,8 @@ namespace {
 constexpr int kMaxN = 1023;
 constexpr size_t kPlane = (size_t)kMaxN * kMaxN;          // one nx x ny plane
 constexpr size_t kTw = 2016;                               // complex twiddles of M = 64 .. 2048, M/2 each
-constexpr size_t kScratchDoubles = 2 * kPlane + 2 * 2048;  // work plane (the rest is not used)
 
-static __device__ __align__(256) double g_poisson_scratch[kScratchDoubles];
+static __device__ __align__(256) double g_poisson_scratch[kPlane];  // work plane
 // Twiddles exp(-2 pi i k / M), k < M/2, of M = 64 .. 2048 in this order, as constant data of the
 // library's device code: they are there whichever stream or capture makes the first call. Formed by
 // the compiler: the Taylor series of sine and cosine on [0, pi/4] in pairs of doubles (Dekker, "A

@@ -206,7 +206,7 @@ int hpq_get_counters(hpq_handle* h, int64_t* mg_vcycles, int64_t* slices, int64_
  * allocate device memory when they solve — code running under CUDA stream capture, plugins whose
  * host framework owns the memory pool, real-time loops that must not allocate. f and u are
  * device pointers owned by the caller (u may not alias f); `stream` is a cudaStream_t (NULL =
- * default stream). Nothing is allocated: the temporaries live in a 16.1 MiB device array inside
+ * default stream). Nothing is allocated: the temporaries live in an 8.0 MiB device array inside
  * the library. CUDA loads the library's device code lazily, so the first call on each device
  * commits that array's memory there (and may fail with HPQ_ERR_CUDA if the device is full); it is
  * held until the process exits. Limit: nx, ny of the form 2^k - 1 with 31 <= n <= 1023; larger
