@@ -41,10 +41,9 @@ PUSH_BYTES = {8: 5 * 8 + 1 + 10 * 8, 4: 5 * 4 + 1 + 10 * 4}
 # the first smoothing
 MG_REALS_PER_POINT_VCYCLE = 4.0 / 3.0 * 9.0
 MG_REALS_PER_POINT_FIRST = 9.0
-# DRAM bytes of one k_mg_cluster launch from ncu (255 x 255, FP64, three V-cycles,
-# profiles/k_mg_cluster_255_fp64.md): the hierarchy stays in shared memory during the solve, so DRAM
-# traffic is far below the algorithmic bytes
-MG_NCU_DRAM_BYTES_FP64_255 = 3330000
+# DRAM bytes of one solve from ncu (255 x 255, FP64, three V-cycles: k_mg_cluster_coef and k_mg_cluster): the
+# hierarchy stays in shared memory during the solve, so DRAM traffic is far below the algorithmic bytes
+MG_NCU_DRAM_BYTES_FP64_255 = 3930000
 
 
 def parse():
@@ -224,6 +223,7 @@ def run_ours(args):
     classes = ["plasma_deposit", "beam_deposit", "poisson_psi_ez_bz", "explicit_deposit", "multigrid",
                "plasma_push", "beam_push", "beam_partition"]
     prof = {c: sim.profile(c) for c in classes}
+    mg_kernel = "k_mg_cluster" if sim.profile("multigrid_coefficients")[1] else "k_mg_solve"
     sim.set_profiling(False)
     total_prof = sum(v[0] for v in prof.values())
     dominant = max(prof, key=lambda c: prof[c][0])
@@ -233,7 +233,7 @@ def run_ours(args):
     push_bytes = n_plasma * PUSH_BYTES[elem]
     achieved = push_bytes / (push_ms / 1e3 / max(push_n, 1)) / 1e9 if push_n else 0.0
     counters = sim.counters()
-    # dominant kernel: the persistent multigrid solve (one launch per slice)
+    # dominant kernel: the multigrid solve (k_mg_cluster_coef and k_mg_cluster, or k_mg_solve)
     mg_ms, mg_n = prof["multigrid"]
     vc = counters["mg_vcycles"] / max(counters["slices"], 1)
     mg_bytes = (vc * MG_REALS_PER_POINT_VCYCLE + MG_REALS_PER_POINT_FIRST) * nx * ny * elem
@@ -258,7 +258,7 @@ def run_ours(args):
         "e2e": {"value": e2e_value, "unit": "slices/s", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h},
         "gpu_launches": None,
-        "roofline": {"bound": "hbm", "kernel": "k_mg_cluster" if max(nx, ny) <= 256 else "k_mg_solve", "achieved": mg_achieved, "peak": peak,
+        "roofline": {"bound": "hbm", "kernel": mg_kernel, "achieved": mg_achieved, "peak": peak,
                      "unit": "GB/s", "frac": mg_achieved / peak, "peak_kind": peak_kind,
                      "traffic": (MG_NCU_DRAM_BYTES_FP64_255
                                  if (args.config == "blowout_255" and elem == 8) else None),

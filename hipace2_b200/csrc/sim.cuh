@@ -1490,6 +1490,11 @@ public:
     template <bool CELL, class MGT, class RS>
     void mg_run(MGT& mg, const Slab<RS>& MS, bool prepared = false) {
         if (mg.coop_ok) {
+            if (!prepared && mg.cluster_form(cfg.mg_tol_rel)) {
+                Scope sc(this, "multigrid_coefficients");
+                mg.prepare(st, MS, ctl, cfg.mg_tol_rel);
+                prepared = true;
+            }
             // the whole solve, iterations and decisions included, is one kernel
             mg.template solve_persistent<CELL>(st, MS, ctl, cfg.mg_tol_rel, cfg.mg_tol_abs, cfg.mg_max_iters, prepared);
             return;
@@ -2092,8 +2097,8 @@ public:
                              cfg.do_beam_jz_minus_rho ? S.c(C_RHOMJZ).p : nullptr);
         }
         // the multigrid's coefficient hierarchy needs chi alone: beside the Poisson solves and the
-        // explicit deposit
-        const bool prepared = ex && mg.cluster_form(cfg.mg_tol_rel);
+        // explicit deposit (while profiling, where nothing runs beside anything, in the multigrid's class)
+        const bool prepared = ex && !profiling && mg.cluster_form(cfg.mg_tol_rel);
         if (prepared) {
             OnStream on(this, side_begin());
             mg.prepare(st, S, ctl, cfg.mg_tol_rel);

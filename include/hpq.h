@@ -188,7 +188,8 @@ int hpq_salame_log(hpq_handle* h, double* out, int64_t* n);
 int hpq_synchronize(hpq_handle* h);
 /* Per-kernel-class timing with CUDA events on the launching stream (kernel launch mode only).
  * Classes: plasma_deposit, beam_deposit, poisson_psi_ez_bz, explicit_deposit, multigrid,
- * plasma_push, beam_push, beam_partition. hpq_get_profile returns the accumulated device time
+ * multigrid_coefficients (the part of multigrid that builds the coefficient hierarchy, on grids whose
+ * solve runs in clusters), plasma_push, beam_push, beam_partition. hpq_get_profile returns the accumulated device time
  * and number of timed regions since profiling was switched on. */
 int hpq_set_profiling(hpq_handle* h, int on);
 int hpq_get_profile(hpq_handle* h, const char* kernel_class, double* total_ms, int64_t* launches);

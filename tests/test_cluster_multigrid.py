@@ -75,3 +75,18 @@ def test_grids_whose_levels_are_all_split(nx, ny, tol, precision):
 @pytest.mark.parametrize("precision", [hp.PLAIN_FP64, hp.MIXED])
 def test_flat_grids_with_rows_beyond_the_grid(nx, ny, precision):
     test_cluster_form_equals_tile_form(nx, ny, precision, 0.3)
+
+
+def test_profile_counts_the_coefficients_in_the_multigrid_class(monkeypatch):
+    text = deck(63, 63, 1e-4)
+    for form, slices in (("cluster", 12), ("tiles", 0)):
+        monkeypatch.setenv("HPQ_MG", form)
+        g = hp.Hipace(text, graphs=False)
+        g.init_data()
+        g.step(0)
+        g.set_profiling(True)
+        g.step(1)
+        mg, n = g.profile("multigrid")
+        coef, m = g.profile("multigrid_coefficients")
+        assert n == 12 and m == slices and mg > coef >= 0 and (coef > 0) == (slices > 0)
+        g.close()
