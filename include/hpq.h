@@ -59,7 +59,12 @@ int hpq_diag_count(const hpq_handle* h, int64_t* n);
 const char* hpq_create_error(void);
 
 /* Field/plasma arithmetic: HPQ_PLAIN_FP64 (the reference's FP64 path) or HPQ_MIXED (FP32
- * plasma, fields and multigrid; FP64 beam). Call before hpq_init. */
+ * plasma, fields and multigrid; FP64 beam). Call before hpq_init.
+ * With HPQ_MIXED, hipace.MG_tolerance_rel is met up to the rounding of a solution stored in 32
+ * bits. The solver measures its residual as the diagonal times the change that one more sweep would
+ * make, with the sweep's own rounding; the residual of the returned Bx, By evaluated in 64 bits may
+ * be larger by about 2.4e-7 (4 / dx^2 + chi) max|B|, which exceeds 1e-4 of the right-hand side on
+ * fine grids (dx below about 0.02 skin depths). */
 int hpq_set_precision(hpq_handle* h, int mode);
 
 /* Allocate device data and inject the beams; replaces Hipace::InitData()
