@@ -1577,6 +1577,8 @@ public:
     // solve (tolerances below kRefineTol)
     ClPlan<R> cl;
     ClPlan<double> cl64;
+    ClSeat cl_seat;
+    bool cl_coop = false;       // no seat: cooperative launch
     ClNorm* cl_slot = nullptr;  // ClArgs::slot
     void* cl_coef = nullptr;                // ClArgs::coef
 
@@ -1599,6 +1601,7 @@ public:
             // (both components' clusters have to be resident: they exchange norms)
             if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 2) { cudaGetLastError(); continue; }
             pl.ok = true;
+            pl.places = n;
             return;
         }
     }
@@ -1624,6 +1627,9 @@ public:
         const size_t bytes = std::max(cl.ok ? cl.a.cs * (size_t)cl.a.coef_elems * sizeof(R) : 0,
                                       cl64.ok ? cl64.a.cs * (size_t)cl64.a.coef_elems * sizeof(double) : 0);
         if (bytes) {
+            int dev = 0;
+            HPQ_CUDA(cudaGetDevice(&dev));
+            cl_coop = !cl_seat.take(dev, std::min(cl.ok ? cl.places : 1 << 30, cl64.ok ? cl64.places : 1 << 30));
             HPQ_CUDA(cudaMalloc(&cl_slot, 6 * kClMaxBlocks * sizeof(ClNorm)));
             HPQ_CUDA(cudaMalloc(&cl_coef, bytes));
             HPQ_CUDA(cudaMemset(cl_coef, 0, bytes));
@@ -1671,11 +1677,11 @@ public:
         cudaLaunchConfig_t cfg{};
         cudaLaunchAttribute at[2];
         cluster_config(cfg, at, A.cs, pl.smem, st);
-        // both clusters resident or neither: each waits for the other's norms, and the clusters of other
-        // handles may hold the room of one of them
-        at[1].id = cudaLaunchAttributeCooperative;
-        at[1].val.cooperative = 1;
-        cfg.numAttrs = 2;
+        if (cl_coop) {  // both clusters resident or neither
+            at[1].id = cudaLaunchAttributeCooperative;
+            at[1].val.cooperative = 1;
+            cfg.numAttrs = 2;
+        }
         HPQ_CUDA(cudaLaunchKernelEx(&cfg, k_mg_cluster<R, RS, CELL>, A, cluster_view(S, C_BX, C_BY), cluster_view(S, C_SY, C_SX)));
         HPQ_LAUNCH_CHECK();
     }
@@ -1868,6 +1874,7 @@ public:
         coarse.garena = nullptr;
         if (trace) cudaFree(trace);
         trace = nullptr;
+        cl_seat.give();
         if (cl_slot) cudaFree(cl_slot);
         if (cl_coef) cudaFree(cl_coef);
         cl_slot = nullptr;

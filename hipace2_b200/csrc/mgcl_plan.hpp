@@ -5,6 +5,9 @@
 
 #include <algorithm>
 #include <cstddef>
+#include <map>
+#include <mutex>
+#include <set>
 #include <type_traits>
 #include <vector>
 
@@ -118,6 +121,49 @@ HPQ_HD inline int cl_coarse_row(int row, int base, int crp) {
     return c < crp ? c : crp;
 }
 
+// Solvers of this process, by device, whose two clusters are launched without a guarantee that both become
+// resident. Each cluster waits for the other's norms, so such solvers could stop one another only if single
+// halves held every place: with fewer solvers than places at least one place is left for a partner.
+// A solver that would be one too many launches cooperatively (mg.cuh). (Not all do: ncu cannot
+// profile a cooperative launch with clusters.)
+class ClSeat {
+public:
+    ClSeat() = default;
+    ClSeat(const ClSeat&) = delete;
+    ClSeat& operator=(const ClSeat&) = delete;
+    ~ClSeat() { give(); }
+    // false: no seat, launch cooperatively. places: clusters of this solver that an idle GPU holds
+    bool take(int device, int places) {
+        give();
+        std::lock_guard<std::mutex> lock(mutex());
+        std::multiset<int>& taken = seats()[device];
+        const int fewest = taken.empty() ? places : std::min(places, *taken.begin());
+        if ((int)taken.size() + 1 >= fewest) return false;
+        taken.insert(places);
+        device_ = device;
+        places_ = places;
+        return true;
+    }
+    void give() {
+        if (device_ < 0) return;
+        std::lock_guard<std::mutex> lock(mutex());
+        std::multiset<int>& taken = seats()[device_];
+        taken.erase(taken.find(places_));
+        device_ = -1;
+    }
+
+private:
+    static std::mutex& mutex() {
+        static std::mutex* m = new std::mutex;  // (never destroyed: handles may outlive static objects)
+        return *m;
+    }
+    static std::map<int, std::multiset<int>>& seats() {
+        static auto* s = new std::map<int, std::multiset<int>>;
+        return *s;
+    }
+    int device_ = -1, places_ = 0;
+};
+
 // Clusters tried in this order: a whole component in one block where it fits (63^2 in double): a sweep
 // then ends with a block barrier (45 cycles) instead of a cluster barrier (500); else the largest
 // cluster. A level runs in block 0 where its points there cost less than a cluster barrier, as far as
@@ -130,6 +176,7 @@ struct ClPlan {
     bool ok = false;
     ClArgs<R> a{};
     size_t smem = 0;
+    int places = 0;  // clusters of this plan that an idle GPU holds
 
     // planes of every level for clusters of cs blocks, levels of at most `own` points in block 0
     static bool layout(ClArgs<R>& A, size_t& smem, const std::vector<MGLev>& lev, double dx, double dy, int cs,

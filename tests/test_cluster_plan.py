@@ -89,6 +89,22 @@ int main() {
             if (cl_norm_arrived(half, tag) || cl_norm_arrived(half, tag + 2)) ++bad, std::printf("half a norm\n");
         }
     }
+    // seats: fewer solvers than the places of each of them
+    {
+        auto expect = [&](bool got, bool want, const char* what) { if (got != want) ++bad, std::printf("seats: %s\n", what); };
+        ClSeat s[8], other, few, one;
+        for (int i = 0; i < 8; ++i) expect(s[i].take(0, 7), i < 6, "seven places");
+        expect(other.take(1, 7), true, "another device");
+        s[2].give();
+        s[2].give();
+        expect(few.take(0, 3), false, "fewer places than solvers");
+        expect(s[7].take(0, 7), true, "a seat given back");
+        for (ClSeat& x : s) x.give();
+        expect(few.take(0, 2), true, "two places, alone");
+        expect(one.take(0, 148), false, "beside a solver with two places");
+        { ClSeat gone; expect(gone.take(2, 2), true, "taken"); }
+        expect(one.take(2, 2), true, "given back when destroyed");
+    }
     std::printf("%ld plans, %ld faults\n", plans, bad);
     return bad != 0 || plans < 10000;
 }
