@@ -246,9 +246,10 @@ struct SmoothSmem {
 // Both components of a point pair sit in one thread's registers, by colour e = (i + j) & 1: a sweep
 // updates u[.][.][e] from u[.][.][1 - e] of the thread's own rows and pair, and reads only the
 // pair's outer neighbour and the rows beyond its strip from shared memory (rows with even columns
-// first, so that threads read consecutive words). Shared-memory traffic bounds the sweeps: the form
-// that kept rhs, diagonal and all neighbours there, two words apart, moved 4 times as much
-// (1023^2 in double: 58 and 52 us for the two level-0 passes of a V-cycle; the whole solve of a slice took
+// first, so that threads read consecutive words). What bounds it now is the block barrier of each
+// sweep, then the global loads that open a tile (ncu at 1023^2 in double: stalls 9.4 and 5.3 per issue,
+// L1 and shared memory 32 %). Shared-memory traffic bound the form that kept rhs, diagonal and all
+// neighbours there, two words apart, and moved 4 times as much (1023^2 in double: 58 and 52 us for the two level-0 passes of a V-cycle; the whole solve of a slice took
 // 677 us and takes 479, in single precision 508 and 437; 2047^2 single 1415 and 1352). A colour sweep reads
 // the other colour only, so the guess is loaded for colour 1 alone (the first sweep replaces
 // colour 0), and after the last sweep the residual of colour 1 is zero up to rounding: the norm

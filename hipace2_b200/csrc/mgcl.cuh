@@ -24,8 +24,9 @@
 // stored there with even columns first, so that consecutive threads touch consecutive words.
 #pragma once
 
-// Measured on a B200, per V-cycle against the tile form: 57 -> 28 us at 255^2 and 28 -> 13 us at 63^2 (double);
-// per slice at 255^2 192 -> 117 us double, 158 -> 95-99 us mixed.
+// Measured on a B200, per V-cycle against the tile form as it then was: 57 -> 28 us at 255^2 and 28 -> 13 us
+// at 63^2 (double). Per slice at 255^2, the coefficient kernel's 26 us (beside the Poisson solves outside a
+// profile) included: 192 -> 148 us double, 158 -> 130 us mixed; at 63^2 with 7 V-cycles 213 -> 146 us.
 //
 // (included by mg.cuh, whose barrier polls it uses; levels and shared-memory plan: mgcl_plan.hpp)
 
@@ -657,12 +658,11 @@ struct ClSolve {
 };
 
 template <class R>
-__device__ __forceinline__ void cl_levels_to_shared(const ClArgs<R>& P, ClLev<R>* slev, unsigned elems) {
+__device__ __forceinline__ void cl_levels_to_shared(const ClArgs<R>& P, ClLev<R>* slev) {
     static_assert(sizeof(ClLev<R>) % 4 == 0, "copied by words");
     const int* src = reinterpret_cast<const int*>(P.lev);
     int* dst = reinterpret_cast<int*>(slev);
     for (int t = threadIdx.x; t < (int)(sizeof(ClLev<R>) / 4) * P.nl; t += kClThreads) dst[t] = src[t];
-    (void)elems;
 }
 
 // Coefficient hierarchy of a solve, one cluster: restricts the coefficient, inverts the diagonals,
@@ -676,7 +676,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_mg_cluster_coef(const __grid_
     const int cs = P.cs, rank = (int)blockIdx.x;
     R* sm = reinterpret_cast<R*>(cl_smem);
     using S = ClSolve<R, CELL>;
-    cl_levels_to_shared(P, slev, 0);
+    cl_levels_to_shared(P, slev);
     int4* z = reinterpret_cast<int4*>(cl_smem);
     for (unsigned t = threadIdx.x; t < P.celems * sizeof(R) / 16; t += kClThreads) z[t] = make_int4(0, 0, 0, 0);
     if (rank == 0 && threadIdx.x < 6 * kClMaxBlocks) P.slot[threadIdx.x] = ClNorm{};
@@ -758,7 +758,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
                          (uint32_t)__cvta_generic_to_shared(cl_smem)),
                      "l"(P.coef + (size_t)rank * P.coef_elems), "r"(copied), "r"(copy_bar) : "memory");
     }
-    cl_levels_to_shared(P, slev, 0);
+    cl_levels_to_shared(P, slev);
     {
         int4* z = reinterpret_cast<int4*>(cl_smem);
         for (unsigned t = P.coef_elems * sizeof(R) / 16 + threadIdx.x; t < P.elems * sizeof(R) / 16; t += kClThreads)

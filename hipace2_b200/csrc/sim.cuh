@@ -533,8 +533,10 @@ public:
         // others (whole steps on a B200 against the SIMT sine GEMMs: the 64^2 predictor-corrector
         // linear wake 255 vs 337 us per slice, the three solves of 384 x 320 115 vs 345 us; the GEMMs,
         // O(n^3), were not faster anywhere from 48 to 1200). Single precision takes the Bluestein FFT
-        // below 128 (transform length 512; 64^2 97 vs 109 us per slice) and the tensor-core sine GEMMs
-        // (TF32x3) above, up to 1023^2 (256^2 176 vs 197, 600^2 1340 vs 1713).
+        // below 128 (64^2 97 vs 109 us per slice) and the tensor-core sine GEMMs (TF32x3) from there on,
+        // at every size: solves of a one-iteration predictor-corrector slice 56 vs 74 us at 256^2 (where the
+        // transform length doubles; 52 vs 46 at 200^2), 146 vs 244 at 600^2, 330 vs 1161 at 1200^2, 1379
+        // vs 1979 at 2000^2.
         // HPQ_DST=tc / tc_bf16 (BF16x3 tensor-core GEMMs) / fft / gemm (SIMT sine GEMMs on every
         // grid, cross-checks) forces a form
         const char* env = getenv("HPQ_DST");
