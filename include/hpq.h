@@ -63,8 +63,8 @@ const char* hpq_create_error(void);
  * With HPQ_MIXED, hipace.MG_tolerance_rel is met up to the rounding of a solution stored in 32
  * bits. The solver measures its residual as the diagonal times the change that one more sweep would
  * make, with the sweep's own rounding; the residual of the returned Bx, By evaluated in 64 bits may
- * be larger by about 2.4e-7 (4 / dx^2 + chi) max|B|, which exceeds 1e-4 of the right-hand side on
- * fine grids (dx below about 0.02 skin depths). */
+ * be larger by up to 2.4e-7 (2 / dx^2 + 2 / dy^2 + chi) |B|, which on fine grids can be more than
+ * 1e-4 of the right-hand side. */
 int hpq_set_precision(hpq_handle* h, int mode);
 
 /* Allocate device data and inject the beams; replaces Hipace::InitData()
